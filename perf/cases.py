@@ -204,3 +204,54 @@ def tolerance(case):
     # 2-norm errors seen against the same arithmetic in float64; about four times that is stated
     return {"gqa": {"rel": 1e-2}, "mla": {"rel": 1.2e-2}, "oproj": {"rel": 7e-3}, "combine": {"rel": 7e-3},
             "exchange": {"rel": 7e-3}, "step": {"rel": 1.2e-2}}[case["op"]]
+
+
+def _combine64(o, lse):
+    """LSE-weighted sum over the leading dimension, and the LSE of the whole."""
+    o, lse = o.double(), lse.double()
+    return (torch.softmax(lse, 0).unsqueeze(-1) * o).sum(0), torch.logsumexp(lse, 0)
+
+
+def _gqa64(q, k, v, rows, n, scale):
+    """One sequence: ``q [Hq, d]``, ``k`` / ``v`` ``[pages, page, Hkv, d]``, ``rows`` its pages, ``n`` its tokens."""
+    k, v = (t[rows].flatten(0, 1)[:n].double().transpose(0, 1) for t in (k, v))           # [Hkv, n, d]
+    s = q.double().view(k.shape[0], -1, q.shape[-1]) @ k.transpose(1, 2) * scale
+    return (torch.softmax(s, -1) @ v).reshape(q.shape), torch.logsumexp(s, -1).reshape(-1)
+
+
+def exact(case, seed):
+    """What ``run`` returns, from plain torch in float64."""
+    s = prepare(case, seed)
+    op = case["op"]
+    if op == "gqa":
+        k, v = (t.transpose(1, 2) if s["layout"] == "HND" else t for t in (s["k"], s["v"]))
+        each = [_gqa64(s["q"][b], k, v, s["table"][b, :-(-n // case["page"])].long(), n, 1.0 / math.sqrt(128))
+                for b, n in enumerate(s["lens"].tolist())]
+        o, lse = (torch.stack(t) for t in zip(*each))
+        return o, lse / math.log(2.0) if s["base2"] else lse
+    if op == "mla":
+        outs, lses = [], []
+        for b, n in enumerate(s["lens"].tolist()):
+            rows = s["table"][b, :-(-n // case["page"])].long()
+            c = s["ckv"][rows].flatten(0, 1)[:n].double().view(n, 4, 128)
+            c = (c * s["scales"][rows].flatten(0, 1)[:n].double().unsqueeze(-1)).view(n, 512)
+            kpe = s["kpe"][rows].flatten(0, 1)[:n].double()
+            x = (s["q_nope"][b].double() @ c.t() + s["q_pe"][b].double() @ kpe.t()) * s["scale"]
+            outs.append(torch.softmax(x, -1) @ c)
+            lses.append(torch.logsumexp(x, -1))
+        return torch.stack(outs), torch.stack(lses)
+    if op == "oproj":
+        w = prepare(dict(case, packed=False), seed)["w"]
+        return s["x"].double() @ w.double().t()
+    if op == "combine":
+        o, lse = (s["o"], s["lse"]) if s["layout"] == "NBHD" else (s["o"].transpose(0, 1), s["lse"].transpose(0, 1))
+        out, g = _combine64(o, lse)
+        return (out, g) if s["return_lse"] else out
+    if op == "exchange":
+        out, g = _combine64(s["o"], s["lse"])                       # rank r keeps the r-th part of the heads
+        return tuple(torch.stack(t.chunk(s["cp"], dim=1)) for t in (out, g))
+    stack = s["stack"]                                              # the step returns its last layer's output
+    k, v = stack.k_cache[-1].transpose(1, 2), stack.v_cache[-1].transpose(1, 2)
+    o = torch.stack([_gqa64(q, k, v, stack.block_table[b].long(), case["ctx"], 1.0 / math.sqrt(128))[0]
+                     for b, q in enumerate(s["q"][-1].cuda())])
+    return (o.flatten(1) @ stack.w_o[-1].double().t()).cpu()
