@@ -87,7 +87,8 @@ struct MlaDecodeParams {
   unsigned long long* prof;      // lockstep kernel only, optional [ctas][8] clock64 sums of thread 0: waits, dequantise,
                                  // Q K^T, softmax (+ rescale), P store + P V issue, tiles, all clocks of the tile loop
   int B, page_size, ctas;
-  int variant;                   // 0: all warps in lockstep; 1: producer warps + math warps (warp-specialised)
+  int variant;                   // 0: all warps in lockstep; 1: producer warps + math warps (warp-specialised);
+                                 // 2: clusters of two CTAs (`ctas` is even, pieces merged by a second kernel)
   float scale;
   int lse_base2;
   unsigned long long timeout_ns;
@@ -96,6 +97,8 @@ constexpr int kMlaMaxCtas = 296;
 inline size_t mla_part_o_floats(int ctas) { return (size_t)ctas * 2 * 128 * 512; }
 inline size_t mla_part_lse_floats(int ctas) { return (size_t)ctas * 2 * 128; }
 int mla_pick_ctas(int B, int max_seq_len, int sm_count);
+int mla_pair_pick_ctas(int B, int max_seq_len, int sm_count);
+cudaError_t launch_mla_decode_pair(const MlaDecodeParams& p, bool pdl, cudaStream_t stream);
 cudaError_t launch_mla_decode(const MlaDecodeParams& p, bool pdl, cudaStream_t stream);
 
 }  // namespace helix

@@ -190,7 +190,7 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
 }
 
 
-constexpr int kMlaDefaultVariant = 1;   // warp-specialised
+constexpr int kMlaDefaultVariant = 2;   // clusters of two CTAs
 
 // ---- MLA fp8 paged decode attention -----------------------------------------------------------------
 std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch::Tensor q_pe, torch::Tensor ckv,
@@ -222,8 +222,16 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   torch::Tensor o = torch::empty({B, 128, 512}, q_nope.options());
   torch::Tensor lse = torch::empty({B, 128}, q_nope.options().dtype(torch::kFloat32));
   if (B == 0) return std::make_tuple(o, lse);
+  // HELIX_A2A_MLA_VARIANT: "pair" = clusters of two CTAs, "ws" = producer warps + math warps, "lockstep" = all warps in
+  // lockstep
+  const char* v = std::getenv("HELIX_A2A_MLA_VARIANT");
+  const int variant = !v ? kMlaDefaultVariant
+                         : std::string(v) == "lockstep" ? 0 : std::string(v) == "ws" ? 1 : kMlaDefaultVariant;
+  const int longest = (int)std::max<int64_t>(max_seq_len, 1);
   int nc = ctas > 0 ? (int)std::min<int64_t>(ctas, helix::kMlaMaxCtas)
-                    : helix::mla_pick_ctas(B, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
+           : variant == 2 ? helix::mla_pair_pick_ctas(B, longest, helix::device_sm_count())
+                          : helix::mla_pick_ctas(B, longest, helix::device_sm_count());
+  if (variant == 2) nc = std::max(nc / 2 * 2, 2);
   Scratch& sc = scratch_for(q_nope.device(), (int64_t)B + 1024, (int64_t)helix::mla_part_o_floats(nc),
                             (int64_t)helix::mla_part_lse_floats(nc));
   helix::MlaDecodeParams p{};
@@ -245,11 +253,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   p.scale = (float)scale;
   p.lse_base2 = lse_base2 ? 1 : 0;
   p.timeout_ns = env_timeout_ns();
-  {
-    // HELIX_A2A_MLA_VARIANT: "ws" = producer warps + math warps, "lockstep" = all warps in lockstep
-    const char* v = std::getenv("HELIX_A2A_MLA_VARIANT");
-    p.variant = (v && std::string(v) == "lockstep") ? 0 : (v && std::string(v) == "ws") ? 1 : kMlaDefaultVariant;
-  }
+  p.variant = variant;
   p.prof = nullptr;
   {
     static const bool prof_on = [] { const char* v = std::getenv("HELIX_A2A_MLA_PROF"); return v && std::string(v) == "1"; }();

@@ -1123,6 +1123,7 @@ int mla_pick_ctas(int B, int max_seq_len, int sm_count) {
 }
 
 cudaError_t launch_mla_decode(const MlaDecodeParams& p, bool pdl, cudaStream_t stream) {
+  if (p.variant == 2) return launch_mla_decode_pair(p, pdl, stream);
   if (p.B <= 0) return cudaSuccess;
   if (p.page_size % kBlk != 0 || p.ctas < 1 || p.ctas > kMlaMaxCtas) return cudaErrorInvalidValue;
   const bool ws = p.variant == 1;
