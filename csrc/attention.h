@@ -26,15 +26,15 @@ struct GqaDecodeParams {
   float* part_o;               // scratch [2 * ctas + max_helper][8][128] fp32: piece slots
   float* part_lse;             // scratch [2 * ctas + max_helper][8]
   // scratch, zero on entry and zero again on exit (gqa_counter_ints(B * Hkv, max_helper) ints):
-  //   [0, P)          blocks of each (sequence, kv head) pair that have been folded into a piece so far
+  //   [0, P)          blocks of the fold that have read the flags of a (sequence, kv head) pair
   //   [P, 2P)         chunks drawn from each pair's dynamic pool          (touched only when dyn_pct > 0)
-  //   [2P]            CTAs that have left the launch                      (touched only when dyn_pct > 0)
   //   [2P + 8, ...)   one flag per helper slot: a piece has been parked there
   int* counters;
   int* error_flag;             // set to a helix::Status code when a bounded wait runs out
   unsigned long long* trace;   // optional [ctas][8] stamps (%globaltimer): entry, first data, end of the fixed share,
                                // exit, end of the last drawn chunk, chunks drawn | pools visited << 32, SM id
   int B, Hq, Hkv, page_size, ctas;
+  int whole;                   // 1: one CTA per (sequence, kv head) pair (grid B * Hkv, `ctas` unused), nothing is split
   // Dynamic tail: of every pair with at least dyn_min_blocks KV blocks, the last dyn_pct percent (rounded down to
   // whole chunks of dyn_chunk blocks) are not part of any CTA's fixed share; CTAs draw them chunk by chunk when
   // their own share is done, so SMs that stream faster end up streaming more.  dyn_pct = 0: fixed shares only.
@@ -60,6 +60,9 @@ constexpr size_t gqa_counter_ints(int pairs, int max_helper) { return (size_t)2 
 
 // number of CTAs that fills the device for this batch (two per SM unless the work is tiny)
 int gqa_pick_ctas(int B, int Hkv, int max_seq_len, int sm_count);
+
+// Sequences so short that a pair is not worth splitting: one CTA per pair.
+bool gqa_whole_pairs(int B, int Hkv, int max_seq_len, int sm_count);
 
 // Dynamic-tail settings for a launch of `ctas` CTAs: fills dyn_pct / dyn_chunk / dyn_min_blocks / max_helper of *p
 // (pct_override / chunk_override < 0: the library's choice; max_helper 0 switches the dynamic tail off).

@@ -168,6 +168,7 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   p.counters = sc.counters.data_ptr<int32_t>();
   p.error_flag = sc.error_flag.data_ptr<int32_t>();
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.page_size = page; p.ctas = sp;
+  p.whole = splits <= 0 && helix::gqa_whole_pairs(B, Hkv, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
   // HELIX_A2A_ATTN_DYN_PCT / HELIX_A2A_ATTN_DYN_CHUNK: share of every long pair that is handed out dynamically
   // (0 = fixed shares only) and the chunk size in 16-token blocks; unset = the library's choice
   helix::gqa_plan_dynamic(&p, (int)std::max<int64_t>(max_seq_len, 1), max_helper, env_int("HELIX_A2A_ATTN_DYN_PCT", -1),

@@ -24,9 +24,11 @@
 //     ldmatrix from the swizzled tile;
 //   * the first loads of the next segment are issued before the epilogue of the current one;
 //   * when a CTA leaves a pair, its warps' partial (max, sum, O) are merged through shared memory
-//     and parked as one normalised piece in scratch memory, unless the CTA saw the whole pair; every
-//     piece adds its block count to the pair's counter, and the CTA whose piece completes the pair
-//     folds all pieces - no second launch, and nobody ever waits for another CTA.
+//     and parked as one normalised piece in scratch memory, unless the CTA saw the whole pair;
+//     a second kernel, chained by programmatic launch, folds the pieces with all SMs;
+//   * short sequences (gqa_whole_pairs) are not split at all: one CTA per pair, no tables, one launch.
+// Measured (B200, launches back to back in a graph): 1 x 131072 tokens 97.3 us with the fold by the pair's last CTA, 91 us
+// with the fold kernel (5.9 TB/s); 1 x 300 tokens 18.6 -> 9.6 us, 16 ragged up to 500 tokens 32.7 -> 11.0 us unsplit.
 // Every mbarrier wait is bounded; on expiry the kernel raises the error flag and leaves.
 #include "attention.h"
 
@@ -49,12 +51,13 @@ constexpr int kStages = 3;
 constexpr int kTileBytes = kBlockTok * kD * 2;        // 4096: one K (or V) block
 constexpr int kStageBytes = 2 * kTileBytes;           // K + V
 constexpr int kSmemPipe = kWarps * kStages * kStageBytes;   // 98304
-constexpr int kMergeBytes = kWarps * 4 * kD * 4;        // 8192: warps' partial O of four heads / piece list of a fold
+constexpr int kMergeBytes = kWarps * 4 * kD * 4;        // 8192: warps' partial O of four heads
 constexpr int kSmemBytes = kSmemPipe + kMergeBytes + 1024;   // + alignment slack
-constexpr int kMaxList = kMergeBytes / 4;               // pieces one fold can list
+constexpr int kMaxList = 2048;                          // pieces one fold can list
 constexpr int kMaxPoolChunks = kMaxList - kGqaMaxCtas;   // chunks one pair's pool may hold: a fold lists at most one piece
                                                         // per CTA plus one per chunk of the pair
 static_assert(kMaxPoolChunks > 0, "the piece list must hold one piece per CTA");
+constexpr int kMinShare = 8, kWholeBlocks = 96, kWholeExtra = 40;      // 16-token blocks, see gqa_pick_ctas
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -82,107 +85,70 @@ __device__ __forceinline__ int ld_relaxed(const int* p) {
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
-  int prev;
-  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(prev) : "l"(p), "r"(v) : "memory");
-  return prev;
+
+// Chunks a pair gives to its pool, `want` being what dyn_pct asks for and hb the helper slots handed out so far.
+// A pair only gets a pool if what stays in the fixed shares is longer than one share.  A CTA's share then
+// never holds such a pair from its first block to its last fixed block, so the share's two piece slots
+// (one for a pair it continues, one for a pair it starts) still suffice, and some share ends inside the pair, so
+// a CTA is there to take up the pool.  (Two shares were the better line while one CTA folded all pieces of a pair;
+// now 24 ragged sequences up to 9000 tokens, 8 kv heads, take 82.6 us with one share and 87.0 with two.)
+__device__ __forceinline__ int pool_chunks(const GqaDecodeParams& p, int nb, int want, long long share_max, int hb) {
+  if (nb - want * p.dyn_chunk <= share_max) return 0;
+  if (hb + want * p.Hkv > p.max_helper || want > kMaxPoolChunks) return 0;    // never more chunks than helper slots
+  return want;
 }
 
-// The CTA whose piece completed a pair folds all pieces listed in s_list (piece slots) into the final output.
-// Warp w folds heads 2w and 2w + 1 together: lanes first share out the pieces' weights, then every lane sums
-// four columns of both heads with sixteen independent 16-byte loads in flight.  Kept out of line so that its
-// registers do not weigh on the streaming loop.
-struct FoldArgs {
-  const float* part_o;
-  const float* part_lse;
-  __nv_bfloat16* o;
-  float* lse;
-  int Hq, lse_base2;
+// Where the pieces of one pair are: CTAs i0 .. i1 stream its fixed part, nc chunks from helper slot hb on form its pool.
+struct PairPlan {
+  int i0, i1, nc, hb;
 };
-constexpr int kFoldBatch = 8;
-__device__ __noinline__ void fold_pieces(FoldArgs p, const int* s_list, int n_pieces, int st_b, int st_kvh, int group,
-                                         int warp, int lane) {
-  // Warp w folds heads 2w and 2w + 1.  Pieces are taken eight at a time: their LSEs and their rows are requested
-  // together (16 + 2 independent loads per lane), so a batch costs ONE round trip to L2; the running maximum is
-  // carried from batch to batch as in an online softmax.  (Sixteen at a time needs so many registers that the
-  // streaming loop of the kernel around this function starts to spill: measured 30 % slower.)
-  const int h0 = warp * 2, h1 = warp * 2 + 1;
-  if (h0 >= group) return;
-  const bool has1 = h1 < group;
-  float M0 = -INFINITY, M1 = -INFINITY, L0 = 0.f, L1 = 0.f;
-  float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int c0 = 0; c0 < n_pieces; c0 += kFoldBatch) {
-    const int nb = min(kFoldBatch, n_pieces - c0);
-    const int my_slot = lane < nb ? s_list[c0 + lane] : 0;
-    float l0 = -INFINITY, l1 = -INFINITY;
-    if (lane < nb) {
-      l0 = __ldcg(p.part_lse + (size_t)my_slot * 8 + h0);
-      if (has1) l1 = __ldcg(p.part_lse + (size_t)my_slot * 8 + h1);
-    }
-    float4 v0[kFoldBatch], v1[kFoldBatch];
-#pragma unroll
-    for (int j = 0; j < kFoldBatch; ++j) {
-      if (j < nb) {
-        const int sl = __shfl_sync(0xffffffffu, my_slot, j);
-        const float4* po = reinterpret_cast<const float4*>(p.part_o + (size_t)sl * 8 * kD);
-        v0[j] = __ldcg(po + h0 * (kD / 4) + lane);
-        if (has1) v1[j] = __ldcg(po + h1 * (kD / 4) + lane);
-      }
-    }
-    float b0 = l0, b1 = l1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {       // lanes beyond the batch hold -inf
-      b0 = fmaxf(b0, __shfl_xor_sync(0xffffffffu, b0, o));
-      b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, o));
-    }
-    const float n0 = fmaxf(M0, b0), n1 = fmaxf(M1, b1);
-    const float s0 = (M0 == -INFINITY) ? 0.f : fast_exp2(M0 - n0);
-    const float s1 = (M1 == -INFINITY) ? 0.f : fast_exp2(M1 - n1);
-    const float w0 = (l0 == -INFINITY) ? 0.f : fast_exp2(l0 - n0);
-    const float w1 = (l1 == -INFINITY) ? 0.f : fast_exp2(l1 - n1);
-    M0 = n0;
-    M1 = n1;
-    L0 = L0 * s0 + w0;
-    L1 = L1 * s1 + w1;
-    a0.x *= s0; a0.y *= s0; a0.z *= s0; a0.w *= s0;
-    a1.x *= s1; a1.y *= s1; a1.z *= s1; a1.w *= s1;
-#pragma unroll
-    for (int j = 0; j < kFoldBatch; ++j) {
-      if (j < nb) {
-        const float x0 = __shfl_sync(0xffffffffu, w0, j);
-        const float x1 = __shfl_sync(0xffffffffu, w1, j);
-        a0.x += x0 * v0[j].x;
-        a0.y += x0 * v0[j].y;
-        a0.z += x0 * v0[j].z;
-        a0.w += x0 * v0[j].w;
-        if (has1) {
-          a1.x += x1 * v1[j].x;
-          a1.y += x1 * v1[j].y;
-          a1.z += x1 * v1[j].z;
-          a1.w += x1 * v1[j].w;
-        }
-      }
+
+// The fold's view of the tables the streaming kernel builds (the same rules; see there).
+__device__ __forceinline__ PairPlan plan_pair(const GqaDecodeParams& p, int b, int kvh, int* s_nb, unsigned short* s_nc,
+                                              long long* s_part) {
+  const int tid = threadIdx.x, cd = p.dyn_chunk, G = p.ctas;
+  const bool dyn_cfg = p.dyn_pct > 0 && cd > 0 && p.B <= kGqaSeqTable && p.max_helper > 0;
+  if (tid < 2) s_part[tid] = 0;
+  __syncthreads();
+  long long all = 0, before = 0;
+  for (int i = tid; i < p.B; i += blockDim.x) {
+    const int nb = blocks_of(p.seq_lens[i]);
+    all += nb;
+    if (i < b) before += nb;
+    if (dyn_cfg) {
+      s_nb[i] = nb;
+      s_nc[i] = (unsigned short)min(dyn_chunks_of(nb, p.dyn_pct, cd, p.dyn_min_blocks), 65535);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    L0 += __shfl_xor_sync(0xffffffffu, L0, o);
-    L1 += __shfl_xor_sync(0xffffffffu, L1, o);
-  }
-  auto store_head = [&](int hg, float M, float L, const float4& a) {
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    const int h = st_kvh * group + hg;
-    uint2 packed;
-    packed.x = pack_bf16(a.x * inv, a.y * inv);
-    packed.y = pack_bf16(a.z * inv, a.w * inv);
-    *reinterpret_cast<uint2*>(p.o + ((int64_t)st_b * p.Hq + h) * kD + lane * 4) = packed;
-    if (lane == 0) {
-      const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
-      p.lse[(int64_t)st_b * p.Hq + h] = p.lse_base2 ? lse2 : lse2 * kLn2;
+  if (before) atomicAdd(reinterpret_cast<unsigned long long*>(&s_part[0]), (unsigned long long)before);
+  if (all) atomicAdd(reinterpret_cast<unsigned long long*>(&s_part[1]), (unsigned long long)all);
+  __syncthreads();
+  PairPlan pl{0, -1, 0, 0};
+  long long start = s_part[0], total = s_part[1];
+  int ns = blocks_of(p.seq_lens[b]);
+  if (dyn_cfg) {
+    const long long share_max = (total * p.Hkv + G - 1) / G + 1;
+    long long fixed = 0;
+    int hb = 0;
+    for (int i = 0; i < p.B; ++i) {
+      const int nb = s_nb[i], nc = pool_chunks(p, nb, s_nc[i], share_max, hb);
+      if (i == b) {
+        start = fixed;
+        pl.nc = nc;
+        pl.hb = hb + kvh * nc;
+        ns = nb - nc * cd;
+      }
+      hb += nc * p.Hkv;
+      fixed += nb - nc * cd;
     }
-  };
-  store_head(h0, M0, L0, a0);
-  if (has1) store_head(h1, M1, L1, a1);
+    total = fixed;
+  }
+  if (ns > 0) {
+    const long long share = max((total * p.Hkv + G - 1) / (long long)G, 1LL), sp0 = start * p.Hkv + (long long)kvh * ns;
+    pl.i0 = (int)(sp0 / share);
+    pl.i1 = (int)((sp0 + ns - 1) / share);
+  }
+  return pl;
 }
 
 // kTrace: the instance that records time stamps (the stamps cost registers the streaming loop needs)
@@ -226,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   const bool dyn_cfg = p.dyn_pct > 0 && cd > 0 && p.B <= kGqaSeqTable && p.max_helper > 0;
   bool dyn_on = false;                           // some pair of this launch really has a pool
   const int n_tab = min(p.B, kGqaSeqTable);
-  for (int i = tid; i < n_tab; i += kThreads) {
+  for (int i = tid; i < (p.whole ? 0 : n_tab); i += kThreads) {
     // (the divisions are done here, one sequence per thread, not in the serial pass below)
     const int nb = blocks_of(p.seq_lens[i]);
     s_nb[i] = nb;
@@ -234,22 +200,15 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   }
   __syncthreads();
   long long total_s = 0;                         // blocks in the fixed shares
-  {
+  if (!p.whole) {
     long long total = 0;
     for (int b = 0; b < n_tab; ++b) total += s_nb[b];
     for (int b = kGqaSeqTable; b < p.B; ++b) total += blocks_of(p.seq_lens[b]);
-    // A pair only gets a pool if what stays in the fixed shares is longer than two shares.  A CTA's share then
-    // never holds such a pair from its first block to its last fixed block, so the share's two piece slots
-    // (one for a pair it continues, one for a pair it starts) still suffice; some share ends inside the pair, so
-    // a CTA is there to take up the pool; and pairs of about a share's length, where nearly every chunk would end
-    // up as a parked piece of its own, keep their fixed shares only (measured slower with pools).
-    const long long share_max = 2 * ((total * Hkv + G - 1) / G);
+    const long long share_max = (total * Hkv + G - 1) / G + 1;
     int hb = 0;
     for (int b = 0; b < n_tab; ++b) {
       const int nb = s_nb[b];
-      int nc = s_nc[b];
-      if (nb - nc * cd <= share_max) nc = 0;
-      if (hb + nc * Hkv > p.max_helper || nc > kMaxPoolChunks) nc = 0;    // never more chunks than helper slots
+      const int nc = pool_chunks(p, nb, s_nc[b], share_max, hb);
       if (tid == 0) {
         s_ncf[b] = (unsigned short)nc;
         s_hb[b] = hb;
@@ -270,10 +229,8 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   const long long g0 = (long long)blockIdx.x * share;
   const long long g1 = min(total_s, g0 + share);
 
-  int* const done_ctr = p.counters;                      // [P]
   int* const pool_ctr = p.counters + (size_t)p.B * Hkv;   // [P]
-  int* const exit_ctr = p.counters + (size_t)2 * p.B * Hkv;
-  int* const helper_flag = exit_ctr + 8;                 // [max_helper]
+  int* const helper_flag = p.counters + (size_t)2 * p.B * Hkv + 8;   // [max_helper]
   const int P = p.B * Hkv;
 
   uint8_t* my_smem = smem + warp * (kStages * kStageBytes);
@@ -292,13 +249,13 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   };
   int cur_b = 0;
   long long base = 0;        // share-space index of block 0 of (cur_b, kvh = 0)
-  while (cur_b < p.B) {
+  while (!p.whole && cur_b < p.B) {
     const long long span = (long long)seq_ns(cur_b) * Hkv;
     if (g0 < base + span) break;
     base += span;
     ++cur_b;
   }
-  long long gcur = g0;
+  long long gcur = p.whole ? g1 : g0;
   auto next_static = [&]() {
     Seg sg;
     sg.valid = false;
@@ -410,9 +367,20 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   };
 
   float* s_o = reinterpret_cast<float*>(smem + kSmemPipe);   // [kWarps][4][kD]: merge buffer, not part of the rings
-  int* s_list = reinterpret_cast<int*>(smem + kSmemPipe);    // the same bytes list a fold's pieces
 
-  Seg cur = next_static();
+  Seg cur;
+  if (p.whole) {                       // CTA = (sequence, kv head) pair, nothing to share out
+    cur.b = blockIdx.x / Hkv;
+    cur.kvh = blockIdx.x % Hkv;
+    cur.seq_len = p.seq_lens[cur.b];
+    cur.n_blocks = blocks_of(cur.seq_len);
+    cur.kb_begin = 0;
+    cur.kb_end = cur.n_blocks;
+    cur.slot = 0;
+    cur.valid = cur.n_blocks > 0;
+  } else {
+    cur = next_static();
+  }
   if (early_kv) {
     // old KV does not depend on the kernel before us: request the first tiles, then wait for it (q does depend).
     // A segment that reaches the newest token waits first: that token's K/V row may still be on its way.
@@ -640,50 +608,8 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
         }
       }
 
-      if (!whole) {
-        // Publish this piece and count its blocks with ONE acquire-release atomic by thread 0 after a CTA
-        // barrier (the barrier orders the other threads' partial stores before it, the release makes
-        // them visible device-wide; the acquire side lets the arrival that completes the pair read
-        // everybody's pieces).
-        const int pair = st_b * Hkv + st_kvh;
-        __syncthreads();
-        if (tid == 0) {
-          if (st_slot >= 2 * G) helper_flag[st_slot - 2 * G] = 1;
-          const int prev = atom_add_acq_rel(done_ctr + pair, st_blocks);
-          s_flag = (prev + st_blocks == st_nb);
-        }
-        __syncthreads();
-        const bool completes = s_flag != 0;
-        if (completes) {
-          // ---- this piece completed the pair: fold all of its pieces ---------------------------------
-          __syncthreads();                    // everybody has read the verdict before s_flag is reused
-          // pieces from the fixed shares: one per CTA whose share overlaps the pair's static blocks
-          const int nc = seq_nc(st_b), ns = st_nb - nc * cd;
-          long long sp0 = 0;
-          for (int bb = 0; bb < st_b; ++bb) sp0 += seq_ns(bb);
-          sp0 = sp0 * Hkv + (long long)st_kvh * ns;
-          const int i0 = (int)(sp0 / share), i1 = (int)((sp0 + ns - 1) / share);
-          const int n_fixed = i1 - i0 + 1;
-          for (int i = tid; i < n_fixed; i += kThreads) s_list[i] = (i0 + i) * 2 + (i == 0 ? 1 : 0);
-          if (tid == 0) s_flag = n_fixed;
-          __syncthreads();
-          // pieces parked by CTAs that helped out of this pair's pool
-          const int hb = nc > 0 ? s_hb[st_b] + st_kvh * nc : 0;
-          for (int c = tid; c < nc; c += kThreads) {
-            if (ld_relaxed(helper_flag + hb + c) != 0) {
-              const int k = atomicAdd(&s_flag, 1);
-              if (k < kMaxList) s_list[k] = 2 * G + hb + c;
-              helper_flag[hb + c] = 0;                     // ready for the next launch
-            }
-          }
-          __syncthreads();
-          const int n_pieces = min(s_flag, kMaxList);
-          fold_pieces(FoldArgs{p.part_o, p.part_lse, p.o, p.lse, Hq, p.lse_base2}, s_list, n_pieces, st_b, st_kvh, group,
-                      warp, lane);
-          if (tid == 0) done_ctr[pair] = 0;   // ready for the next launch
-          __syncthreads();                    // the list is read; the merge buffer may be reused
-        }
-      }
+      // a piece parked in a helper slot is announced to the fold kernel; those of the fixed shares it knows itself
+      if (!whole && tid == 0 && st_slot >= 2 * G) helper_flag[st_slot - 2 * G] = 1;
       // the running state is consumed: a fresh one starts with the next segment
       st_active = false;
       m_run = -INFINITY;
@@ -705,16 +631,6 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
       while (!mbar_try_wait(&full_bar[warp][s], 0) && !mbar_try_wait(&full_bar[warp][s], 1)) {
         if ((++spins & 255u) == 0u && now_ns() > grace) break;
       }
-    }
-  } else if (dyn_on && warp == 0) {
-    // the last CTA to leave re-arms the pools for the next launch: nobody draws or probes any more (every warp
-    // of this CTA is past the loop above; only this warp waits for the atomic)
-    int last = 0;
-    if (lane == 0) last = (atom_add_acq_rel(exit_ctr, 1) == G - 1);
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (last) {
-      for (int i = lane; i < P; i += 32) pool_ctr[i] = 0;
-      if (lane == 0) *exit_ctr = 0;
     }
   }
 
@@ -743,14 +659,116 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   }
 }
 
+// Merges the pieces of every pair that more than one CTA streamed, one launch behind the streaming kernel: it
+// is resident early (its tables are ready before the pieces are) and then has every SM to read them, where a fold by
+// the CTA that finished a pair last had one SM read all of its pieces, eight per round trip, behind an acquire-release
+// atomic that takes ~4 us while HBM is saturated.  Block (pair, y) merges query heads y, y + gridDim.y, ... of
+// the pair's group: warps share out the pieces, lanes the columns.  The last block of a pair clears its pool and flags.
+constexpr int kFoldThreads = 128;
+__global__ void __launch_bounds__(kFoldThreads) gqa_fold_kernel(const __grid_constant__ GqaDecodeParams p) {
+  __shared__ unsigned short s_list[kMaxList];
+  __shared__ float4 s_acc[kFoldThreads / 32 - 1][32];
+  __shared__ float s_red[kFoldThreads / 32];
+  __shared__ int s_n;
+  __shared__ long long s_part[2];
+  __shared__ int s_nb[kGqaSeqTable];
+  __shared__ unsigned short s_nc[kGqaSeqTable];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pair = blockIdx.x, b = pair / p.Hkv, kvh = pair % p.Hkv, group = p.Hq / p.Hkv;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // seq_lens is final here: the streaming kernel waits for its predecessors before it lets this one start, or has
+  // been promised that they do not touch it (kv_stable)
+  const PairPlan pl = plan_pair(p, b, kvh, s_nb, s_nc, s_part);
+  const int n_fixed = pl.i1 - pl.i0 + 1;
+  for (int i = tid; i < n_fixed; i += kFoldThreads) s_list[i] = (unsigned short)((pl.i0 + i) * 2 + (i == 0 ? 1 : 0));
+  if (tid == 0) s_n = n_fixed;
+  __syncthreads();
+  // Every block waits, also one without work: who waits for this launch counts on the streaming kernel being done.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (n_fixed <= 0 || (n_fixed == 1 && pl.nc == 0)) return;          // empty, or written by the CTA that saw all of it
+  int* const helper_flag = p.counters + (size_t)2 * p.B * p.Hkv + 8 + pl.hb;
+  for (int c = tid; c < pl.nc; c += kFoldThreads)
+    if (__ldcg(helper_flag + c) != 0) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(2 * p.ctas + pl.hb + c);
+  __syncthreads();
+  const int n = s_n;
+  if (pl.nc > 0) {
+    if (tid == 0) s_nb[0] = atomicAdd(p.counters + pair, 1) == (int)gridDim.y - 1;
+    __syncthreads();
+    if (s_nb[0]) {                              // every block of the pair has read the flags
+      for (int c = tid; c < pl.nc; c += kFoldThreads) helper_flag[c] = 0;
+      if (tid == 0) {
+        p.counters[(size_t)p.B * p.Hkv + pair] = 0;
+        p.counters[pair] = 0;
+      }
+    }
+  }
+  for (int hg = blockIdx.y; hg < group; hg += gridDim.y) {
+    // weights of the pieces
+    float M = -INFINITY;
+    for (int i = tid; i < n; i += kFoldThreads) M = fmaxf(M, __ldcg(p.part_lse + (size_t)s_list[i] * 8 + hg));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    if (lane == 0) s_red[warp] = M;
+    __syncthreads();
+    M = s_red[0];
+#pragma unroll
+    for (int w = 1; w < kFoldThreads / 32; ++w) M = fmaxf(M, s_red[w]);
+    float L = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int i = warp; i < n; i += kFoldThreads / 32) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p.part_o + ((size_t)s_list[i] * 8 + hg) * kD) + lane);
+      const float l = __ldcg(p.part_lse + (size_t)s_list[i] * 8 + hg), w = l == -INFINITY ? 0.f : fast_exp2(l - M);
+      L += w;
+      acc.x += w * v.x;
+      acc.y += w * v.y;
+      acc.z += w * v.z;
+      acc.w += w * v.w;
+    }
+    __syncthreads();                            // s_red is read
+    if (warp > 0) s_acc[warp - 1][lane] = acc;
+    if (lane == 0) s_red[warp] = L;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int w = 1; w < kFoldThreads / 32; ++w) {
+        const float4 v = s_acc[w - 1][lane];
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+        L += s_red[w];
+      }
+      const float inv = L > 0.f ? 1.f / L : 0.f;
+      const int64_t row = (int64_t)b * p.Hq + kvh * group + hg;
+      *(reinterpret_cast<uint2*>(p.o + row * kD) + lane) = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+      if (lane == 0) {
+        const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
+        p.lse[row] = p.lse_base2 ? lse2 : lse2 * kLn2;
+      }
+    }
+    __syncthreads();                            // s_acc and s_red are free again
+  }
+}
+
 }  // namespace
 
-// Number of CTAs for a launch: two per SM, but never so many that a CTA streams fewer than
-// 32 blocks (its fixed ramp + merge cost is worth about that much streaming).
+// Number of CTAs for a launch: two per SM, but never so many that a CTA streams fewer than 8 blocks (two per warp).
+// With 32 blocks as the limit one sequence of 4000 tokens (8 kv heads) took 19.6 us and four of up to 1000 took
+// 21.6 us; with about 128 CTAs each 17.3 and 15.9 us.
 int gqa_pick_ctas(int B, int Hkv, int max_seq_len, int sm_count) {
   const long long blocks = (long long)std::max(B, 1) * Hkv * std::max((max_seq_len + kBlockTok - 1) / kBlockTok, 1);
-  long long ctas = std::min<long long>(2LL * sm_count, std::max<long long>(blocks / 32, 1));
+  long long ctas = std::min<long long>(2LL * sm_count, std::max<long long>(blocks / kMinShare, 1));
   return (int)std::min<long long>(ctas, kGqaMaxCtas);
+}
+
+// One CTA per pair costs the longest sequence's blocks, a quarter per warp at about 0.35 us each; shares cost their
+// own length the same way and a fold (about 4 us with its launch).  So pairs stay whole while the longest one is no
+// more than kWholeExtra blocks longer than a share would be, and not so long that ragged batches are left with a tail.
+bool gqa_whole_pairs(int B, int Hkv, int max_seq_len, int sm_count) {
+  const long long blocks = blocks_of(std::max(max_seq_len, 1)), slots = 2LL * sm_count;
+  const long long pairs = std::min((long long)std::max(B, 1) * Hkv, slots);
+  return blocks <= kWholeBlocks && blocks * (slots - pairs) <= kWholeExtra * slots;
 }
 
 void gqa_plan_dynamic(GqaDecodeParams* p, int max_seq_len, int max_helper, int pct_override, int chunk_override) {
@@ -789,21 +807,25 @@ cudaError_t launch_gqa_decode(const GqaDecodeParams& p, bool pdl, cudaStream_t s
     if (dev < 64) attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.ctas, 1, 1);
+  cfg.gridDim = dim3(p.whole ? p.B * p.Hkv : p.ctas, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attrs[1];
-  int na = 0;
-  if (pdl) {
-    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
-  cfg.attrs = attrs;
-  cfg.numAttrs = na;
-  return p.trace != nullptr ? cudaLaunchKernelEx(&cfg, gqa_decode_kernel<true>, p)
-                            : cudaLaunchKernelEx(&cfg, gqa_decode_kernel<false>, p);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaError_t e = p.trace != nullptr ? cudaLaunchKernelEx(&cfg, gqa_decode_kernel<true>, p)
+                                     : cudaLaunchKernelEx(&cfg, gqa_decode_kernel<false>, p);
+  if (e != cudaSuccess || p.whole) return e;
+  // The fold is always chained to this launch; it waits for the whole grid before it reads a piece.
+  const int pairs = p.B * p.Hkv;
+  cfg.gridDim = dim3(pairs, std::max(1, std::min(p.Hq / p.Hkv, 1184 / pairs)), 1);
+  cfg.blockDim = dim3(kFoldThreads, 1, 1);
+  cfg.dynamicSmemBytes = 0;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gqa_fold_kernel, p);
 }
 
 }  // namespace helix

@@ -141,6 +141,7 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
   p.Hkv = kv_heads;
   p.page_size = page_size;
   p.ctas = ctas;
+  p.whole = helix::gqa_whole_pairs(batch, kv_heads, max_seq_len > 0 ? max_seq_len : 1, st->sm_count);
   // fixed shares only: the dynamic tail of the kernel needs more scratch than this array has
   p.dyn_pct = 0;
   p.dyn_chunk = 0;

@@ -1,0 +1,42 @@
+"""GQA decode attention: unsplit short sequences and the fold kernel, against the fp32 oracle and each other."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(lens, hkv, group, page, layout, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    blocks = max(1, max((n + page - 1) // page for n in lens))
+    pages = len(lens) * blocks + 3
+    bt = torch.randperm(pages, generator=gen, device="cuda")[:len(lens) * blocks].view(len(lens), blocks).int()
+    shape = (pages, hkv, page, 128) if layout == "HND" else (pages, page, hkv, 128)
+    k, v = (torch.empty(shape, device="cuda").normal_(generator=gen).bfloat16() for _ in range(2))
+    q = torch.empty(len(lens), hkv * group, 128, device="cuda").normal_(generator=gen).bfloat16()
+    return q, k, v, bt, torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+
+# around one 16-token block, around the longest unsplit sequence (512 tokens), empty sequences, few and many pairs,
+# groups of one to eight heads; splits = 0 leaves the form to the library, the others force shares and the fold
+@pytest.mark.parametrize("lens,hkv,group,page,layout", [
+    ([1], 1, 1, 16, "HND"), ([15, 16, 17, 0], 8, 8, 16, "NHD"), ([300], 8, 8, 16, "HND"), ([511, 512, 64], 2, 4, 32, "NHD"),
+    ([513, 3], 8, 3, 16, "HND"), ([100] * 40 + [0, 1], 8, 8, 64, "HND"), ([2000, 0, 90, 7000], 4, 8, 16, "HND"),
+    ([40, 600] * 150, 2, 8, 16, "HND"), ([20000], 8, 8, 16, "NHD")])
+def test_forms_agree_with_the_oracle(native_built, lens, hkv, group, page, layout):
+    from helix_a2a_b200.ops import attention, reference_math as rm
+    from helix_a2a_b200.ops.oproj import check_compute_status
+    q, k, v, bt, sl = _case(lens, hkv, group, page, layout, len(lens) + hkv)
+    kc, vc = (t if layout == "HND" else t.permute(0, 2, 1, 3) for t in (k, v))
+    o_ref, l_ref = rm.paged_decode_attention_reference(q.cpu(), kc.cpu(), vc.cpu(), bt.cpu(), sl.cpu(), 1 / math.sqrt(128), False)
+    for splits in (0, 1, 3):
+        for _ in range(2):      # the second call also shows that the first one left counters and pools as it found them
+            o, lse = attention.gqa_decode(q, k, v, bt, sl, layout=layout, splits=splits, max_seq_len=max(lens))
+        torch.cuda.synchronize()
+        check_compute_status(q)
+        live = (sl > 0).cpu()
+        # probabilities and the result carry one bf16 rounding each: 2 x 2^-9 of values up to about 4.5
+        assert (o.cpu().float() - o_ref.float()).abs().max() < 2e-2, splits
+        assert (lse.cpu()[live] - l_ref[live]).abs().max() < 1e-3, splits
+        assert torch.isneginf(lse.cpu()[~live]).all()
