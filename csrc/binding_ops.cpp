@@ -296,7 +296,9 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     }
     const int bk = 64 * helix::oproj_pick_atoms(n_pad);
     const int sk_ctas = (int)std::min<int64_t>(sms, (int64_t)(hidden / 128) * ((K + bk - 1) / bk));
-    if (sp <= 0) sp = helix::oproj_pick_splits(hidden, K, sms);
+    const helix::OprojSplitPlan plan = sp == 0 && !streamk ? helix::oproj_pick_split_plan(hidden, K, n_pad, sms)
+                                                           : helix::OprojSplitPlan{0, 0};
+    if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, sms);
     const int64_t part_floats = streamk ? (int64_t)helix::oproj_streamk_partial_floats(sk_ctas, n_pad)
                                         : (sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0);
     Scratch& sc = scratch_for(x.device(), hidden / 128 + 1024, part_floats, 0);
@@ -322,7 +324,9 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
         p.trace = reinterpret_cast<unsigned long long*>(sc.trace.data_ptr());
       }
     }
-    check_cuda(streamk ? helix::launch_oproj_streamk(p, env_pdl(), stream) : helix::launch_oproj(p, env_pdl(), stream),
+    check_cuda(streamk          ? helix::launch_oproj_streamk(p, env_pdl(), stream)
+               : plan.slabs > 0 ? helix::launch_oproj_split(p, plan.slabs, env_pdl(), stream)
+                                : helix::launch_oproj(p, env_pdl(), stream),
                "o_proj launch");
   }
   return y;
@@ -349,7 +353,9 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     torch::Tensor xs = x.narrow(0, t0, nt);
     const int n_pad = (nt + 15) / 16 * 16;
     int sp = (int)splits;
-    if (sp <= 0) sp = helix::oproj_pick_splits(hidden, K, helix::device_sm_count());
+    const helix::OprojSplitPlan plan = sp <= 0 ? helix::oproj_pick_split_plan(hidden, K, n_pad, helix::device_sm_count())
+                                               : helix::OprojSplitPlan{0, 0};
+    if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, helix::device_sm_count());
     Scratch& sc = scratch_for(x.device(), hidden / 128 + 1024,
                               sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0, 0);
     helix::OprojParams p{};
@@ -366,7 +372,8 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     p.stages = helix::oproj_pick_stages(n_pad);
     p.atoms = helix::oproj_pick_atoms(n_pad);
     p.timeout_ns = env_timeout_ns();
-    check_cuda(helix::launch_oproj(p, env_pdl(), stream), "o_proj (packed) launch");
+    check_cuda(plan.slabs > 0 ? helix::launch_oproj_split(p, plan.slabs, env_pdl(), stream) : helix::launch_oproj(p, env_pdl(), stream),
+               "o_proj (packed) launch");
   }
   return y;
 }

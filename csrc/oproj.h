@@ -49,4 +49,12 @@ inline size_t oproj_streamk_partial_floats(int ctas, int n_pad) { return (size_t
 bool oproj_streamk_pays(int hidden, int K, int n_pad, int sm_count);
 cudaError_t launch_oproj_streamk(const OprojParams& p, bool pdl, cudaStream_t stream);
 
+// Split variant: CTAs of one or two 128-row slabs, fine K splits, partials summed by a second kernel.
+// Scratch: partial [splits][n_pad][hidden] fp32 (as large as the plain kernel's).
+struct OprojSplitPlan {
+  int slabs, splits;     // slabs 0: the plain kernel is the better one
+};
+OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int n_pad, int sm_count);
+cudaError_t launch_oproj_split(const OprojParams& p, int slabs, bool pdl, cudaStream_t stream);
+
 }  // namespace helix

@@ -255,6 +255,195 @@ __global__ void __launch_bounds__(kSkThreads, 1) oproj_streamk_kernel(const __gr
   if (warp == 1) tmem_dealloc(tmem_d, tmem_cols);
 }
 
+// ---- split variant: fine K splits, one or two slabs per CTA, partials summed by a second kernel ------------------
+// What bounds a call with more than a handful of tokens is what each SM can take in (about 58 GB/s), not HBM and not
+// the tensor cores: every slab's CTA re-reads all of x (at 256 tokens two bytes of x per byte of W), and with split K
+// the last CTA of a slab read all partials of the plain kernel alone (8 splits x 256 tokens x 128 rows: a megabyte).
+// Here K is cut so that nearly every SM has a CTA; with kSlabs = 2 a CTA owns 256 rows of W with two accumulators in
+// tensor memory, so each x tile in shared memory is used twice; partials are [split][token][hidden] fp32 and
+// oproj_split_fold_kernel sums them with all SMs.  oproj_pick_split_plan says which form a call takes.
+// Measured (packed weights, launches back to back in a graph, plain kernel -> this one): hidden 7168, K 8192, 200 tokens
+// 59.3 -> 40.5 us, 64 tokens 34.6 -> 29.1; hidden 2048, K 8192, 64 tokens 32.6 -> 15.5; hidden 4096, K 4096, 32 tokens
+// 17.6 -> 13.7.  Below 32 tokens and with at most two splits the two are level, and the plain kernel is one launch.
+// kSlabs * 4 warps: warp 0 feeds the ring (`atoms` 64-wide K atoms per stage), warp 1 issues the MMAs, and each group of
+// four warps reads one slab's accumulator out.
+constexpr int kSplitMaxStages = 8;
+constexpr int kSplitMinTokens = 32;
+
+__host__ __device__ __forceinline__ int split_atom_bytes(int slabs, int n_pad) { return (slabs * kBM + n_pad) * kAtomK * 2; }
+
+template <int kSlabs>
+__global__ void __launch_bounds__(kSlabs * 128, 1) oproj_split_kernel(const __grid_constant__ OprojParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kSplitMaxStages], empty_bar[kSplitMaxStages], acc_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
+
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int stages = p.stages, atoms = p.atoms, n_atoms = p.K / kAtomK;
+  const int a0 = (int)((long long)blockIdx.y * n_atoms / p.splits), a1 = (int)((long long)(blockIdx.y + 1) * n_atoms / p.splits);
+  const int count = (a1 - a0 + atoms - 1) / atoms;     // stages' worth of K, >= 1: no more splits than atoms
+  const uint32_t w_bytes = kBM * kAtomK * 2, x_bytes = (uint32_t)p.n_pad * kAtomK * 2;      // multiples of 1024
+  const uint32_t slab_bytes = w_bytes * atoms, stage_bytes = kSlabs * slab_bytes + x_bytes * atoms;
+  uint32_t acc_col = 32;
+  while ((int)acc_col < p.n_pad) acc_col <<= 1;
+  const uint32_t tmem_cols = kSlabs * acc_col;
+
+  if (tid == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_bar, 1);
+    mbar_fence_init();
+    s_abort = 0;
+    tma_prefetch_desc(&p.w_map);
+    tma_prefetch_desc(&p.x_map);
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_d = tmem_slot;
+  const unsigned long long deadline = now_ns() + p.timeout_ns;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  if (warp == 0 && lane == 0) {
+    // ---------------- producer ----------------
+    auto load_w = [&](int i) {
+      const int s = i % stages, first = a0 + i * atoms, na = min(atoms, a1 - first);
+      mbar_expect_tx(&full_bar[s], (uint32_t)na * (kSlabs * w_bytes + x_bytes));
+#pragma unroll
+      for (int m = 0; m < kSlabs; ++m) {
+        uint8_t* dst = smem + (size_t)s * stage_bytes + m * slab_bytes;
+        const int slab = kSlabs * blockIdx.x + m;
+        if (p.w_packed != nullptr)
+          bulk_load_1d(dst, p.w_packed + ((size_t)slab * p.packed_atoms + first) * w_bytes, na * w_bytes, &full_bar[s]);
+        else
+          for (int a = 0; a < na; ++a) tma_load_2d(dst + a * w_bytes, &p.w_map, &full_bar[s], (first + a) * kAtomK, slab * kBM);
+      }
+    };
+    auto load_x = [&](int i) {
+      const int s = i % stages, first = a0 + i * atoms, na = min(atoms, a1 - first);
+      for (int a = 0; a < na; ++a)
+        tma_load_2d(smem + (size_t)s * stage_bytes + kSlabs * slab_bytes + a * x_bytes, &p.x_map, &full_bar[s],
+                    (first + a) * kAtomK, 0);
+    };
+    // weights first: they do not depend on the kernel before us
+    const int pre = min(stages, count);
+    for (int i = 0; i < pre; ++i) load_w(i);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = 0; i < pre; ++i) load_x(i);
+    for (int i = pre; i < count; ++i) {
+      if (!mbar_wait(&empty_bar[i % stages], (uint32_t)((i / stages - 1) & 1), deadline)) {
+        fail(p, &s_abort);
+        break;
+      }
+      load_w(i);
+      load_x(i);
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ---------------- MMA issuer ----------------
+    const uint32_t idesc = umma_idesc_bf16(kBM, p.n_pad);
+    bool ok = true;
+    for (int i = 0; i < count; ++i) {
+      const int s = i % stages, na = min(atoms, a1 - a0 - i * atoms);
+      if (!mbar_wait(&full_bar[s], (uint32_t)((i / stages) & 1), deadline)) {
+        fail(p, &s_abort);
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t w_addr = smem_u32(smem + (size_t)s * stage_bytes), x_addr = w_addr + kSlabs * slab_bytes;
+      for (int a = 0; a < na; ++a)
+#pragma unroll
+        for (int m = 0; m < kSlabs; ++m)
+#pragma unroll
+          for (int k = 0; k < kAtomK / 16; ++k)
+            umma_bf16(tmem_d + m * acc_col, umma_desc_k_sw128(w_addr + m * slab_bytes + a * w_bytes + k * 32),
+                      umma_desc_k_sw128(x_addr + a * x_bytes + k * 32), idesc, (i | a | k) != 0);
+      umma_commit(&empty_bar[s]);
+    }
+    if (ok) umma_commit(&acc_bar);
+  }
+  __syncwarp();
+  // ---------------- epilogue (all warps) ----------------
+  int good = 1;
+  if (lane == 0) {                                     // only one lane polls: a failed wait must not split the warp
+    unsigned spins = 0;
+    while (!mbar_try_wait(&acc_bar, 0)) {
+      if ((++spins & 63u) == 0u && (*reinterpret_cast<volatile int*>(&s_abort) || now_ns() > deadline)) {
+        good = 0;
+        break;
+      }
+    }
+    if (!good) fail(p, &s_abort);
+  }
+  good = __shfl_sync(0xffffffffu, good, 0);
+  tc_fence_after_sync();
+  if (good) {
+    const int m = warp >> 2, quad = warp & 3;
+    const int col = (kSlabs * blockIdx.x + m) * kBM + quad * 32 + lane;     // TMEM lane = row of the W slab
+    const uint32_t acc = tmem_d + ((uint32_t)(quad * 32) << 16) + m * acc_col;
+    float* part = p.partial + (size_t)blockIdx.y * p.n_pad * p.hidden + col;
+    auto store = [&](int c0, const uint32_t (&v)[16]) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int tok = c0 + j;
+        if (tok < p.tokens) {
+          if (p.splits == 1) p.y[(int64_t)tok * p.y_stride + col] = __float2bfloat16(__uint_as_float(v[j]));
+          else __stcg(part + (size_t)tok * p.hidden, __uint_as_float(v[j]));
+        }
+      }
+    };
+    uint32_t v[2][16];
+    int c0 = 0;
+    for (; c0 + 32 <= p.n_pad; c0 += 32) {
+      tmem_ld_32x32b_x16(acc + (uint32_t)c0, v[0]);
+      tmem_ld_32x32b_x16(acc + (uint32_t)c0 + 16, v[1]);
+      tmem_ld_wait();
+      store(c0, v[0]);
+      store(c0 + 16, v[1]);
+    }
+    if (c0 < p.n_pad) {
+      tmem_ld_32x32b_x16(acc + (uint32_t)c0, v[0]);
+      tmem_ld_wait();
+      store(c0, v[0]);
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_d, tmem_cols);
+}
+
+// y[token][column] = sum of the splits' partials; thread = four columns, block row = token
+__global__ void __launch_bounds__(256) oproj_split_fold_kernel(const __grid_constant__ OprojParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int quad = blockIdx.x * blockDim.x + threadIdx.x, tok = blockIdx.y;
+  if (quad * 4 >= p.hidden) return;
+  const float4* src = reinterpret_cast<const float4*>(p.partial + (size_t)tok * p.hidden) + quad;
+  const size_t step = (size_t)p.n_pad * p.hidden / 4;
+  float4 acc = __ldcg(src);
+#pragma unroll 4
+  for (int s = 1; s < p.splits; ++s) {
+    const float4 v = __ldcg(src + s * step);
+    acc.x += v.x;
+    acc.y += v.y;
+    acc.z += v.z;
+    acc.w += v.w;
+  }
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
+  uint2 out;
+  out.x = *reinterpret_cast<const uint32_t*>(&lo);
+  out.y = *reinterpret_cast<const uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(p.y + (int64_t)tok * p.y_stride + quad * 4) = out;
+}
+
 }  // namespace
 
 int oproj_pick_atoms(int n_pad) { return n_pad <= 64 ? 4 : (n_pad <= 128 ? 2 : 1); }
@@ -341,6 +530,63 @@ cudaError_t launch_oproj_streamk(const OprojParams& p, bool pdl, cudaStream_t st
   cfg.attrs = attrs;
   cfg.numAttrs = na;
   return cudaLaunchKernelEx(&cfg, oproj_streamk_kernel, p);
+}
+
+// A call's form is the cheapest of {one, two slabs} x K splits that fit the SMs at once, by what bounds the parts: a CTA
+// takes in its share of W and all of x for its K range at 58 GB/s; W arrives at 6 TB/s altogether; partials cost a
+// launch (3 us) and 0.25 us per MB.  The plain kernel (no second launch, four atoms per copy) keeps the calls that
+// it serves without a split, or with few tokens and no more than two.
+OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int n_pad, int sm_count) {
+  OprojSplitPlan best{0, 0};
+  const int plain = oproj_pick_splits(hidden, K, sm_count);
+  if (n_pad < kSplitMinTokens && plain <= 2) return best;
+  float best_us = 1e30f;
+  const int n_atoms = K / kAtomK;
+  for (int slabs = 1; slabs <= 2; ++slabs) {
+    if (hidden % (slabs * kBM) != 0) continue;
+    const int groups = hidden / (slabs * kBM), most = std::min({std::max(sm_count / groups, 1), 16, n_atoms});
+    for (int splits = 1; splits <= most; ++splits) {
+      const float in = (float)((n_atoms + splits - 1) / splits) * split_atom_bytes(slabs, n_pad) / 58e3f;
+      const float w = (float)hidden * K * 2 / 6e6f * std::max(1.f, (float)sm_count * 0.75f / (groups * splits));
+      const float us = std::max(in, w) + (splits > 1 ? 3.f + 0.25e-6f * splits * n_pad * hidden * 4 : 0.f);
+      if (us < best_us) best_us = us, best = OprojSplitPlan{slabs, splits};
+    }
+  }
+  if (best.slabs == 1 && best.splits == 1) best.slabs = 0;      // what the plain kernel does, with larger stages
+  return best;
+}
+
+cudaError_t launch_oproj_split(const OprojParams& p, int slabs, bool pdl, cudaStream_t stream) {
+  if (p.tokens <= 0) return cudaSuccess;
+  if ((slabs != 1 && slabs != 2) || p.hidden % (slabs * kBM) != 0 || p.K % kAtomK != 0 || p.n_pad % 16 != 0 || p.n_pad < 16 ||
+      p.n_pad > 256 || p.tokens > p.n_pad || p.splits < 1 || p.splits > p.K / kAtomK || (p.splits > 1 && p.partial == nullptr))
+    return cudaErrorInvalidValue;
+  OprojParams q = p;
+  const int atom = split_atom_bytes(slabs, p.n_pad);
+  q.atoms = atom <= 28 * 1024 ? 2 : 1;
+  q.stages = std::min(kSplitMaxStages, 222 * 1024 / (q.atoms * atom));
+  const int smem = q.stages * q.atoms * atom + 1024;
+  auto kernel = slabs == 2 ? oproj_split_kernel<2> : oproj_split_kernel<1>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(p.hidden / (slabs * kBM), p.splits, 1);
+  cfg.blockDim = dim3(slabs * 128, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kernel, q);
+  if (e != cudaSuccess || p.splits == 1) return e;
+  // always chained to this launch: it waits for the whole grid before it reads anything
+  cfg.gridDim = dim3((p.hidden / 4 + 255) / 256, p.tokens, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.dynamicSmemBytes = 0;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, oproj_split_fold_kernel, q);
 }
 
 }  // namespace helix
