@@ -12,15 +12,22 @@
 //   * tensor memory: O 128 x 256 (256 columns), Q (144 columns, the A operand of every Q K^T straight from tensor
 //     memory), P (32 columns, the A operand of P V) and S (64 columns): 496 of 512, and shared memory is left to
 //     four tiles of 64 tokens;
-//   * a CTA's Q K^T is a partial sum over its dims: it goes to the other CTA as fp32 through distributed shared
-//     memory (st.async, completion counted on the receiver's mbarrier), both add the same two numbers and run the
-//     same softmax, so nothing else has to be agreed on: fp addition commutes, hence bit-identical decisions.
-// Roles per CTA (17 warps): 0..7 softmax (thread = one head x 32 tokens), 8..15 dequantisation fed by register
-// prefetch two tiles ahead, 16 issues the MMAs.  The MMA queue runs Q K^T two tiles ahead of P V, so the partial
-// sums' way to the peer and the softmax are covered.
+//   * a CTA's Q K^T is a partial sum over its dims.  CTA r finishes the 64 heads [64 r, 64 r + 64): it receives the other
+//     CTA's fp32 partial scores of these through distributed shared memory (st.async, completion counted on the
+//     receiver's mbarrier), runs their softmax and returns the bf16 probabilities (and the factor by which O has to
+//     shrink, 1 almost always), which the other CTA puts next to its own as the A operand of its P V.
+// Roles per CTA (20 warps): warp 0 issues the MMAs (the oldest warp, so that busier ones do not keep it waiting; the
+// whole warp walks the loop and one lane issues, which lets the operands stay in uniform registers); warps 4..7 and 8..11
+// are two groups that take tiles in turn (thread = one head; two warps of a group finish this CTA's heads, two forward
+// the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19 dequantise, fed by register prefetch two tiles ahead.  The MMA queue
+// runs Q K^T two tiles ahead of P V.
 // Pieces of a sequence are merged by a second small kernel (mla_pair_fold_kernel) with all SMs.
-// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 666 -> 606 us, 16 ragged
-// sequences up to 17000 tokens 251 -> 139 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
+// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 662 -> 445 us, 16 ragged
+// sequences up to 17000 tokens 253 -> 88 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
+// On the way there: one softmax group whose threads exchanged all partial scores, 606 us with buffer credits and 495
+// without; two groups 478; each CTA finishing half of the heads 445.  A third of the warps more (32 tokens a thread)
+// lost: 520.  A tile takes about 3000 cycles, of which the tensor pipe is busy 2100: an MMA with A in tensor memory and
+// N = 64 takes 83 cycles (32 of them arithmetic), P V's with N = 256 170.
 // Every wait is bounded; on expiry the error flag is raised, tensor memory is released and the kernel returns.
 #include "attention.h"
 
@@ -44,11 +51,14 @@ constexpr int kSlots = 4;
 constexpr int kSubBytes = kTile * 128;                 // [64 tokens x 64 dims] bf16, 128-byte swizzle
 constexpr int kLatBytes = (kDo / 64) * kSubBytes;      // 32768
 constexpr int kSlotBytes = kLatBytes + kTile * 64;     // + rope [64 tokens x 32 dims], 64-byte swizzle: 36864
-constexpr int kXBytes = kH * kTile * 4;                // partial scores of a tile: 32768
-constexpr int kSmem = kSlots * kSlotBytes + 2 * kXBytes + 1024;
-constexpr int kSmWarps = 8, kDqWarps = 8;
+constexpr int kHo = kH / 2;                            // heads that one CTA finishes
+constexpr int kXBytes = kHo * kTile * 4;               // their partial scores of a tile from the peer: 16384
+constexpr int kPxBytes = kHo * kTile * 2;              // the peer's probabilities of the other heads: 8192
+constexpr int kSmem = kSlots * kSlotBytes + 2 * kXBytes + 2 * kPxBytes + 1024;
+constexpr int kGroupWarps = 4, kSmWarps = 2 * kGroupWarps, kDqWarps = 8;
 constexpr int kSmThreads = kSmWarps * 32;
-constexpr int kThreads = (kSmWarps + kDqWarps + 4) * 32;      // the last warpgroup only holds the issuing thread
+constexpr int kFirstSm = 4, kFirstDq = kFirstSm + kSmWarps;  // warps 1..3 only fill the issuing warp's warpgroup
+constexpr int kThreads = (kFirstDq + kDqWarps) * 32;
 constexpr uint32_t kColO = 0, kColQ = 256, kColP = 400, kColS = 448;
 constexpr int kSeqTable = 512;
 constexpr int kSmBar = 1;
@@ -99,15 +109,35 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&v)[
       "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem desc], A with two bf16 of the K index per 32-bit column
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
-  const uint32_t acc = accumulate ? 1u : 0u;
+__device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&v)[32]) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+      "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]),
+      "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[tmem] (+)= A[tmem] * B[smem desc], A with two bf16 of the K index per 32-bit column; the whole warp comes here and
+// the lane with `issue` set issues
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate,
+                                             uint32_t issue) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_by(uint64_t* bar, uint32_t issue) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(smem_u32(bar)), "r"(issue)
       : "memory");
 }
 // K-major operand of 64-byte rows with the 64-byte swizzle, 8-row groups 512 bytes apart
@@ -124,28 +154,23 @@ __device__ __forceinline__ void st_async_f32x4(uint32_t addr, uint32_t bar, floa
                ::"r"(addr), "r"(bar), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
                : "memory");
 }
+__device__ __forceinline__ void st_async_u32x4(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2,%3,%4,%5}, [%1];"
+               ::"r"(addr), "r"(bar), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void st_async_f32(uint32_t addr, uint32_t bar, float v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %2, [%1];" ::"r"(addr), "r"(bar), "f"(v) : "memory");
+}
+__device__ __forceinline__ uint4 lds_u32x4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 lds_f32x4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned long long deadline_ns) {
-  unsigned spins = 0;
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((++spins & 255u) == 0u && now_ns() > deadline_ns) return false;
-  }
 }
 __device__ __forceinline__ void bar_sync_named(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ int bar_or_named(int id, int n, int pred) {
@@ -163,11 +188,15 @@ __device__ __forceinline__ int bar_or_named(int id, int n, int pred) {
   return r;
 }
 
-// Two e4m3 bytes in the high bytes of the 16-bit halves of x -> the same two numbers times 2^-120 as bf16: the byte
-// s.eeee.mmm moved to s.000.0eeee.mmm.0000, subnormals included.
-__device__ __forceinline__ __nv_bfloat162 e4m3x2_as_bf16x2(uint32_t x) {
-  const uint32_t bits = ((x >> 4) & 0x07FF07FFu) | (x & 0x80008000u);
-  return *reinterpret_cast<const __nv_bfloat162*>(&bits);
+// Four e4m3 bytes -> the same numbers times 2^-120 as bf16: a byte s.eeee.mmm moved to s.000.0eeee.mmm.0000 IS that
+// bf16, subnormals included.  Bytes 0 and 2 land in the first word, 1 and 3 in the second (fewer moves than neighbours
+// together); dims 4 i + 1 and 4 i + 2 therefore change places in the tile, in Q on its way to tensor memory (swap_mid)
+// and back again where O is read out.
+__device__ __forceinline__ void e4m3x4_as_bf16x4(uint32_t w, __nv_bfloat162& even, __nv_bfloat162& odd) {
+  const uint32_t e = ((w << 4) & 0x07F007F0u) | ((w << 8) & 0x80008000u);
+  const uint32_t o = ((w >> 4) & 0x07F007F0u) | (w & 0x80008000u);
+  even = *reinterpret_cast<const __nv_bfloat162*>(&e);
+  odd = *reinterpret_cast<const __nv_bfloat162*>(&o);
 }
 
 // The tiles of all sequences form one line, sequence after sequence; cluster c takes tiles [c * chunk, (c + 1) * chunk).
@@ -208,14 +237,15 @@ struct Fetch {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     mla_pair_kernel(const __grid_constant__ MlaDecodeParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t kv_full[kSlots], kv_free[kSlots], s_full, s_free, x_full[2], x_free[2], p_full, q_full, drain;
+  __shared__ __align__(8) uint64_t kv_full[kSlots], kv_free[kSlots], s_full[2], s_free, x_full[2], px_full[2], inv_full, p_full, q_full, m_bar[kGroupWarps], drain;
   __shared__ uint32_t tmem_slot;
-  __shared__ float s_red[2][kH];
+  __shared__ float s_m[kH], s_l[2][kH], s_alpha[2][kHo], s_inv[kHo];
   __shared__ int s_seq[kSeqTable];
   __shared__ int s_total;
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* x_buf = smem + kSlots * kSlotBytes;
+  uint8_t* px_buf = x_buf + 2 * kXBytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank(), peer = rank ^ 1u;
   const int cluster = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
@@ -225,19 +255,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       mbar_init(&kv_full[i], kDqWarps);
       mbar_init(&kv_free[i], 1);            // tcgen05.commit behind the tile's P V
     }
-    mbar_init(&s_full, 1);                  // tcgen05.commit behind a tile's Q K^T
-    mbar_init(&s_free, kSmWarps);
-    for (int i = 0; i < 2; ++i) {
+    mbar_init(&s_free, kGroupWarps);
+    for (int i = 0; i < 2; ++i) {           // one set per softmax group: a wait must never be two phases ahead
+      mbar_init(&s_full[i], 1);             // tcgen05.commit behind a tile's Q K^T
       mbar_init(&x_full[i], 1);             // + the bytes of the peer's partial scores
-      mbar_init(&x_free[i], kSmWarps);      // arrivals from the peer's softmax warps
+      mbar_init(&px_full[i], 1);            // + the bytes of the peer's probabilities and factors
     }
-    mbar_init(&p_full, kSmWarps);
+    for (int i = 0; i < kGroupWarps; ++i) mbar_init(&m_bar[i], 1);
+    mbar_init(&inv_full, 1);                // + the bytes of the peer's 1 / sum, once per segment
+    mbar_init(&p_full, kGroupWarps);
     mbar_init(&q_full, kSmWarps);
     mbar_init(&drain, 1);
     s_total = 0;
     mbar_fence_init();
   }
-  if (warp == kSmWarps + kDqWarps) {
+  if (warp == 0) {
     tmem_alloc(&tmem_slot, 512);
     tmem_relinquish();
   }
@@ -270,16 +302,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   bool ok = true;
   uint32_t gt = 0;                          // tiles this CTA has been through: fixes slots, buffers and phases
 
-  if (warp < kSmWarps) {
+  if (warp >= kFirstSm && warp < kFirstDq) {
     // =========================== softmax ===========================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
-    const int half = warp >> 2, h = 32 * (warp & 3) + lane;
-    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);     // this warp's lanes of the tensor memory
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    const int quad = warp & 3, h = 32 * quad + lane;
+    const uint32_t grp = (uint32_t)(warp - kFirstSm) / kGroupWarps;     // this group takes tiles n with n % 2 == grp
+    const uint32_t tq = tmem + ((uint32_t)(32 * quad) << 16);           // this warp's lanes of the tensor memory
     const float sl2 = p.scale * kLog2e;
     const float2 sl22 = make_float2(sl2, sl2);
     // an address of this CTA's shared memory plus `to_peer` is the same place in the other CTA
     const uint32_t to_peer = map_to_cta(smem_u32(smem), peer) - smem_u32(smem);
-    const uint32_t x_mine = smem_u32(x_buf) + (uint32_t)(half * 8 * kH + h) * 16u;
+    const bool mine = (uint32_t)(quad >> 1) == rank;                    // this CTA finishes these heads
+    const uint32_t hh = (uint32_t)h & (kHo - 1);
+    const uint32_t x_row = smem_u32(x_buf) + grp * kXBytes + hh * 16u, px_row = smem_u32(px_buf) + grp * kPxBytes + hh * 16u;
+    uint32_t n_seg = 0;
 
     while (ok && walk.next(s_seq, p, seg)) {
       const bool whole = seg.count == seg.n_tiles;
@@ -287,14 +323,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       {
         const uint8_t* qn = reinterpret_cast<const uint8_t*>(p.q_nope + ((int64_t)seg.b * kH + h) * kDn + rank * kDo);
         const uint8_t* qr = reinterpret_cast<const uint8_t*>(p.q_pe + ((int64_t)seg.b * kH + h) * kDr + rank * (kDr / 2));
-        // 9 groups of 16 columns (64 bytes per head): the halves take every other one
-        for (int gq = half; gq < 9; gq += 2) {
+        // 9 pieces of 16 columns (64 bytes per head): the groups take every other one
+        for (int gq = grp; gq < 9; gq += 2) {
           const uint4* src = reinterpret_cast<const uint4*>(gq < 8 ? qn + gq * 64 : qr);
           uint32_t v[16];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint4 t = __ldg(src + j);
             v[4 * j] = t.x, v[4 * j + 1] = t.y, v[4 * j + 2] = t.z, v[4 * j + 3] = t.w;
+          }
+          if (gq < 8) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {            // dims 4 i + 1 and 4 i + 2 change places, as in the tile
+              const uint32_t lo = v[j], hi = v[j + 1];
+              v[j] = __byte_perm(lo, hi, 0x5410);
+              v[j + 1] = __byte_perm(lo, hi, 0x7632);
+            }
           }
           tmem_st_x16(tq + kColQ + 16 * gq, v);
         }
@@ -304,110 +348,124 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (lane == 0) mbar_arrive(&q_full);
       }
 
-      float2 cur[16], nxt[16];
-      // own partial scores of tile i out of tensor memory (scaled), and on their way to the peer
-      auto fetch_and_send = [&](uint32_t n, float2 (&s)[16]) {
-        if (!mbar_wait(&s_full, n & 1, deadline)) ok = false;
+      // The maximum in use is per head and shared by the groups through s_m: whoever takes tile n picks it up after
+      // tile n - 1 has been through (m_bar) and passes it on.  m_mine is the one that l_run refers to.
+      // No credits are needed: the scores of tile n + 2 are sent by a warp that has the probabilities of tile n complete,
+      // which were sent after the scores of tile n had been read; and the other way round.
+      float m_mine = -INFINITY, l_run = 0.f;
+      for (int i = (int)((gt ^ grp) & 1u); i < seg.count; i += 2) {
+        const uint32_t n = gt + i, use = n >> 1;         // `use`: how often this group's exchange buffers have been used
+        // partial scores out of tensor memory, scaled
+        if (!mbar_wait(&s_full[grp], use & 1, deadline)) ok = false;
         tc_fence_after_sync();
-        uint32_t v[32];
-        tmem_ld_x32(tq + kColS + 32 * half, v);
-        tmem_ld_wait();
+        float2 s[32];
+        {
+          uint32_t v[2][32];
+          tmem_ld_x32(tq + kColS, v[0]);
+          tmem_ld_x32(tq + kColS + 32, v[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            s[j] = mul2(make_float2(__uint_as_float(v[j >> 4][2 * (j & 15)]), __uint_as_float(v[j >> 4][2 * (j & 15) + 1])), sl22);
+        }
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_free);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) s[j] = mul2(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), sl22);
-        if (tid == 0) mbar_expect_tx(&x_full[n & 1], kXBytes);
-        if (n >= 2 && ok && !mbar_wait_cluster(&x_free[n & 1], ((n >> 1) - 1) & 1, deadline)) ok = false;
-        if (ok) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            st_async_f32x4(x_mine + to_peer + (n & 1) * kXBytes + j * (kH * 16), smem_u32(&x_full[n & 1]) + to_peer, s[2 * j],
-                           s[2 * j + 1]);
-        }
-      };
-
-      float m_used = -INFINITY, l_run = 0.f;
-      fetch_and_send(gt, cur);
-      // A thread whose wait ran out goes on (its data is garbage) until the next vote, where all leave together.
-      for (int i = 0; i < seg.count; ++i) {
-        const uint32_t n = gt + i;
-        if (i + 1 < seg.count) fetch_and_send(n + 1, nxt);
-        if (ok && !mbar_wait(&x_full[n & 1], (n >> 1) & 1, deadline)) ok = false;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float4 x = lds_f32x4(x_mine + (n & 1) * kXBytes + j * (kH * 16));
-          cur[2 * j] = add2(cur[2 * j], make_float2(x.x, x.y));
-          cur[2 * j + 1] = add2(cur[2 * j + 1], make_float2(x.z, x.w));
-        }
-        __syncwarp();
-        if (lane == 0 && ok) mbar_arrive_remote(smem_u32(&x_free[n & 1]) + to_peer);
-        // tokens past the end of the sequence (last tile only)
-        const int live = seg.seq_len - (seg.t_begin + i) * kTile - 32 * half;
-        if (live < 32) {
+        uint32_t pk[32];
+        float alpha = 1.f;
+        if (mine) {
+          if ((quad & 1) == 0 && lane == 0) mbar_expect_tx(&x_full[grp], kXBytes);
+          if (!mbar_wait(&x_full[grp], use & 1, deadline)) ok = false;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            if (2 * j >= live) cur[j].x = -INFINITY;
-            if (2 * j + 1 >= live) cur[j].y = -INFINITY;
+            const float4 x = lds_f32x4(x_row + j * (kHo * 16));
+            s[2 * j] = add2(s[2 * j], make_float2(x.x, x.y));
+            s[2 * j + 1] = add2(s[2 * j + 1], make_float2(x.z, x.w));
           }
-        }
-        float mx = fmaxf(cur[0].x, cur[0].y);
+          // tokens past the end of the sequence (last tile only)
+          const int live = seg.seq_len - (seg.t_begin + i) * kTile;
+          if (live < kTile) {
 #pragma unroll
-        for (int j = 1; j < 16; ++j) mx = fmaxf(mx, fmaxf(cur[j].x, cur[j].y));
-        // The running maximum is only re-applied when some head's grew by more than 2^8, so O is rarely rescaled
-        // (always at a segment's first tile, where there is nothing to rescale yet).
-        if (bar_or_named(kSmBar, kSmThreads, (!ok || i == 0 || mx > m_used + kRescaleThreshold) ? 1 : 0)) {
-          s_red[half][h] = mx;
-          if (bar_or_named(kSmBar, kSmThreads, ok ? 0 : 1)) {
-            ok = false;
-            break;
-          }
-          mx = fmaxf(mx, s_red[half ^ 1][h]);
-          float alpha = 1.f;
-          if (mx > m_used + kRescaleThreshold || m_used == -INFINITY) {
-            const float m_new = fmaxf(m_used, mx);
-            alpha = m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new);
-            l_run *= alpha;
-            m_used = m_new;
-          }
-          if (i > 0) {
-            // every P V issued so far has to be complete before O is touched
-            if (!mbar_wait(&kv_free[(n - 1) % kSlots], ((n - 1) / kSlots) & 1, deadline)) ok = false;
-            tc_fence_after_sync();
-            for (int c0 = 0; c0 < 128; c0 += 16) {
-              uint32_t v[16];
-              tmem_ld_32x32b_x16(tq + kColO + 128 * half + c0, v);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
-              tmem_st_x16(tq + kColO + 128 * half + c0, v);
+            for (int j = 0; j < 32; ++j) {
+              if (2 * j >= live) s[j].x = -INFINITY;
+              if (2 * j + 1 >= live) s[j].y = -INFINITY;
             }
-            tmem_st_wait();
           }
-          bar_sync_named(kSmBar, kSmThreads);       // s_red may be written again
-        }
-        const float m_neg = m_used == -INFINITY ? 0.f : -m_used;
-        const float2 mn2 = make_float2(m_neg, m_neg);
-        uint32_t pk[16];
-        float2 sum = make_float2(0.f, 0.f);
+          float mx[4];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float2 d = add2(cur[j], mn2);
-          const float2 e = make_float2(fast_exp2(d.x), fast_exp2(d.y));
-          sum = add2(sum, e);
-          pk[j] = pack_bf16(e.x, e.y);
+          for (int j = 0; j < 4; ++j) mx[j] = fmaxf(s[j].x, s[j].y);
+#pragma unroll
+          for (int j = 4; j < 32; ++j) mx[j & 3] = fmaxf(mx[j & 3], fmaxf(s[j].x, s[j].y));
+          const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+          // The maximum is only moved when a head's grew by more than 2^8, so O is rarely rescaled
+          // (always at a segment's first tile, where there is nothing to rescale yet).
+          if (n >= 1 && !mbar_wait(&m_bar[quad], (n - 1) & 1, deadline)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const float m = i == 0 ? -INFINITY : s_m[h];
+          const bool move = top > m + kRescaleThreshold || m == -INFINITY;
+          const float m_new = move ? fmaxf(m, top) : m;
+          if (move) {
+            s_m[h] = m_new;
+            alpha = m == -INFINITY ? 0.f : fast_exp2(m - m_new);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&m_bar[quad]);
+          st_async_f32(smem_u32(&s_alpha[grp][hh]) + to_peer, smem_u32(&px_full[grp]) + to_peer, alpha);
+          if (m_new != m_mine) {
+            l_run = m_mine == -INFINITY ? 0.f : l_run * fast_exp2(m_mine - m_new);
+            m_mine = m_new;
+          }
+          const float m_neg = m_new == -INFINITY ? 0.f : -m_new;
+          const float2 mn2 = make_float2(m_neg, m_neg);
+          float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float2 d = add2(s[j], mn2);
+            const float2 e = make_float2(fast_exp2(d.x), fast_exp2(d.y));
+            sum = add2(sum, e);
+            pk[j] = pack_bf16(e.x, e.y);
+            if ((j & 3) == 3)
+              st_async_u32x4(px_row + to_peer + (j >> 2) * (kHo * 16), smem_u32(&px_full[grp]) + to_peer, pk[j - 3], pk[j - 2],
+                             pk[j - 1], pk[j]);
+          }
+          l_run += sum.x + sum.y;
+        } else {
+          if ((quad & 1) == 0 && lane == 0) mbar_expect_tx(&px_full[grp], kPxBytes + kHo * 4);
+          if (ok) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              st_async_f32x4(x_row + to_peer + j * (kHo * 16), smem_u32(&x_full[grp]) + to_peer, s[2 * j], s[2 * j + 1]);
+          }
+          if (!mbar_wait(&px_full[grp], use & 1, deadline)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          alpha = s_alpha[grp][hh];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint4 v = lds_u32x4(px_row + j * (kHo * 16));
+            pk[4 * j] = v.x, pk[4 * j + 1] = v.y, pk[4 * j + 2] = v.z, pk[4 * j + 3] = v.w;
+          }
         }
-        l_run += sum.x + sum.y;
-        // P has one buffer: the P V of the tile before has to be complete
-        if (n >= 1 && ok && !mbar_wait(&kv_free[(n - 1) % kSlots], ((n - 1) / kSlots) & 1, deadline)) ok = false;
+        // P has one buffer, and O may only be touched between P V products: the one of the tile before is complete
+        if (n >= 1) ok = __all_sync(0xffffffffu, mbar_wait(&kv_free[(n - 1) % kSlots], ((n - 1) / kSlots) & 1, deadline));
+        if (!ok) break;
         tc_fence_after_sync();
-        tmem_st_x16(tq + kColP + 16 * half, pk);
+        if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+          for (int c0 = 0; c0 < kDo; c0 += 16) {
+            uint32_t v[16];
+            tmem_ld_32x32b_x16(tq + kColO + c0, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
+            tmem_st_x16(tq + kColO + c0, v);
+          }
+        }
+        tmem_st_x32(tq + kColP, pk);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) cur[j] = nxt[j];
       }
 
       // ---- O of the segment: normalise, write the result or a piece --------------------------------------
@@ -418,46 +476,62 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         break;
       }
       tc_fence_after_sync();
-      s_red[half][h] = l_run;
-      bar_sync_named(kSmBar, kSmThreads);
-      const float L = s_red[0][h] + s_red[1][h];
-      const float inv = L > 0.f ? 1.f / L : 0.f;
-      const float lse2 = L > 0.f ? m_used + log2f(L) : -INFINITY;
+      float inv, lse2 = 0.f;
+      if (mine) {
+        const float m_used = s_m[h];
+        s_l[grp][h] = m_mine == -INFINITY ? 0.f : l_run * fast_exp2(m_mine - m_used);
+        bar_sync_named(kSmBar, kSmThreads);
+        const float L = s_l[0][h] + s_l[1][h];
+        inv = L > 0.f ? 1.f / L : 0.f;
+        lse2 = L > 0.f ? m_used + log2f(L) : -INFINITY;
+        if (grp == 0) st_async_f32(smem_u32(&s_inv[hh]) + to_peer, smem_u32(&inv_full) + to_peer, inv);
+      } else {
+        if (grp == 0 && (quad & 1) == 0 && lane == 0) mbar_expect_tx(&inv_full, kHo * 4);
+        bar_sync_named(kSmBar, kSmThreads);
+        if (!mbar_wait(&inv_full, n_seg & 1, deadline)) ok = false;      // the vote at the end of the segment acts on it
+        inv = s_inv[hh];
+      }
+      ++n_seg;
       // slot 1: the piece that starts its sequence; a cluster holds at most one piece of each kind
       const size_t slot = (size_t)cluster * 2 + (seg.t_begin == 0 ? 1 : 0);
-      const int col = (int)rank * kDo + 128 * half;
+      const int col = (int)rank * kDo + 128 * grp;
       for (int c0 = 0; c0 < 128; c0 += 16) {
         uint32_t v[16];
-        tmem_ld_32x32b_x16(tq + kColO + 128 * half + c0, v);
+        tmem_ld_32x32b_x16(tq + kColO + 128 * grp + c0, v);
         tmem_ld_wait();
-        if (whole) {
-          uint32_t o16[8];
+        float o[16];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o16[j] = pack_bf16(__uint_as_float(v[2 * j]) * inv, __uint_as_float(v[2 * j + 1]) * inv);
+        for (int j = 0; j < 16; ++j)                     // columns 4 i + 1 and 4 i + 2 change places again
+          o[j] = __uint_as_float(v[(j & 3) == 1 ? j + 1 : (j & 3) == 2 ? j - 1 : j]) * inv;
+        if (whole) {
           uint4* dst = reinterpret_cast<uint4*>(p.o + ((int64_t)seg.b * kH + h) * kDn + col + c0);
-          dst[0] = make_uint4(o16[0], o16[1], o16[2], o16[3]);
-          dst[1] = make_uint4(o16[4], o16[5], o16[6], o16[7]);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            dst[j] = make_uint4(pack_bf16(o[8 * j], o[8 * j + 1]), pack_bf16(o[8 * j + 2], o[8 * j + 3]),
+                                pack_bf16(o[8 * j + 4], o[8 * j + 5]), pack_bf16(o[8 * j + 6], o[8 * j + 7]));
         } else {
           float4* dst = reinterpret_cast<float4*>(p.part_o + (slot * kH + h) * kDn + col + c0);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            dst[j] = make_float4(__uint_as_float(v[4 * j]) * inv, __uint_as_float(v[4 * j + 1]) * inv,
-                                 __uint_as_float(v[4 * j + 2]) * inv, __uint_as_float(v[4 * j + 3]) * inv);
+          for (int j = 0; j < 4; ++j) dst[j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         }
       }
-      if (rank == 0 && half == 0) {
+      if (mine && grp == 0) {
         if (whole) p.lse[(int64_t)seg.b * kH + h] = p.lse_base2 ? lse2 : lse2 * kLn2;
         else p.part_lse[slot * kH + h] = lse2;
       }
       tc_fence_before_sync();
-      bar_sync_named(kSmBar, kSmThreads);           // O and s_red are free for the next segment
+      // O, s_m, s_l and s_inv are free for the next segment
+      if (bar_or_named(kSmBar, kSmThreads, ok ? 0 : 1)) {
+        ok = false;
+        break;
+      }
       gt += seg.count;
     }
     if (!ok && lane == 0) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
-  } else if (warp < kSmWarps + kDqWarps) {
+  } else if (warp >= kFirstDq) {
     // =========================== dequantisation ===========================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-    const int w8 = warp - kSmWarps;
+    const int w8 = warp - kFirstDq;
     // Eight consecutive lanes (one phase of a 16-byte shared-memory access) hold four chunks of an even row and the
     // four of the odd row below: their swizzled stores fall in all eight 16-byte bank groups.
     const int row_lo = 2 * w8 + ((lane & 7) >> 2);                 // row of a 16-token unit
@@ -467,6 +541,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const float* scl_src = p.scales + 2 * rank + (c >> 3);
     const __nv_bfloat16* rope_src = p.kpe + rank * (kDr / 2) + rc * 8;
 
+    const int page_shift = (p.page_size & (p.page_size - 1)) == 0 ? __ffs(p.page_size) - 1 : -1;
     // the tile whose page ids have been requested: lane u (mod 4) holds the ones of 16-token unit u
     int tile_left = 0, tile = 0, nx_page = 0, nx_in = 0, nx_live = 0;
     auto advance = [&]() {
@@ -480,7 +555,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       }
       // a unit past the end of the sequence reads its last unit again: masked, but inside the block table
       const int tok = min(tile * kTile + (lane & 3) * kUnit, (seg.seq_len - 1) / kUnit * kUnit);
-      const int pg = tok / p.page_size;
+      const int pg = page_shift >= 0 ? tok >> page_shift : tok / p.page_size;
       nx_page = p.block_table[(int64_t)seg.b * p.bt_stride + pg];
       nx_in = tok - pg * p.page_size;
       nx_live = min(seg.seq_len - tile * kTile, kTile);
@@ -490,14 +565,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     auto load = [&](Fetch& f) {
       f.live = nx_live;
       if (nx_live == 0) return;
-      const int64_t row = (int64_t)nx_page * p.page_size + nx_in;
+      const uint32_t row = (uint32_t)nx_page * (uint32_t)p.page_size + (uint32_t)nx_in;      // fits: a row is 656 bytes
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int64_t g = __shfl_sync(0xffffffffu, row, u) + row_lo;
-        f.lat[u] = ldg_stream(lat_src + g * kDn);
-        f.scl[u] = __ldg(scl_src + g * 4);
+        const uint32_t g = __shfl_sync(0xffffffffu, row, u) + row_lo;
+        f.lat[u] = ldg_stream(lat_src + (size_t)g * kDn);
+        f.scl[u] = __ldg(scl_src + (size_t)g * 4);
       }
-      f.rope = ldg_stream(rope_src + (__shfl_sync(0xffffffffu, row, w8 >> 1) + (rrow & 15)) * kDr);
+      f.rope = ldg_stream(rope_src + (size_t)(__shfl_sync(0xffffffffu, row, w8 >> 1) + (rrow & 15)) * kDr);
       advance();
     };
     auto convert = [&](Fetch& f) {
@@ -515,10 +590,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const uint32_t w[4] = {f.lat[u].x, f.lat[u].y, f.lat[u].z, f.lat[u].w};
         __nv_bfloat162 v[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          v[2 * j] = e4m3x2_as_bf16x2(__byte_perm(w[j], 0u, 0x1404));
-          v[2 * j + 1] = e4m3x2_as_bf16x2(__byte_perm(w[j], 0u, 0x3424));
-        }
+        for (int j = 0; j < 4; ++j) e4m3x4_as_bf16x4(w[j], v[2 * j], v[2 * j + 1]);
         // times scale * 2^120, which is a finite bf16 for all but absurd scales: those take two factors
         if (fabsf(sc) < 64.f) {
           const __nv_bfloat162 k = __float2bfloat162_rn(sc * 1.329227995784916e36f);       // 2^120
@@ -557,27 +629,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (!ok) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
   } else {
     // =========================== MMA issue ===========================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-    if (warp == kSmWarps + kDqWarps && lane == 0) {
-      const uint32_t id_qk = umma_idesc_bf16(kH, kTile);
-      const uint32_t id_pv = umma_idesc_bf16(kH, kDo) | (1u << 16);       // B is MN-major
-      uint32_t n_seg = 0;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if (warp == 0) {
+      constexpr uint32_t id_qk = umma_idesc_bf16(kH, kTile);
+      constexpr uint32_t id_pv = umma_idesc_bf16(kH, kDo) | (1u << 16);       // B is MN-major
+      const uint32_t issue = lane == 0 ? 1u : 0u;
+      const uint32_t td = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint64_t d_lat = umma_desc_k_sw128(smem_u32(smem)), d_rope = umma_desc_k_sw64(smem_u32(smem) + kLatBytes),
+                     d_val = umma_desc_mn_sw128(smem_u32(smem), kSubBytes);
+      // every lane waits, so that the warp stays together and all agree
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, deadline)) != 0; };
+      // byte offsets enter a descriptor in 16-byte units and never carry out of its 14-bit address field
       auto qk = [&](uint32_t n) {
-        if (!mbar_wait(&kv_full[n % kSlots], (n / kSlots) & 1, deadline)) return false;
-        if (n >= 1 && !mbar_wait(&s_free, (n - 1) & 1, deadline)) return false;
+        if (!wait(&kv_full[n % kSlots], (n / kSlots) & 1)) return false;
+        if (n >= 1 && !wait(&s_free, (n - 1) & 1)) return false;
         tc_fence_after_sync();
-        const uint32_t kv = smem_u32(smem) + (n % kSlots) * kSlotBytes;
+        const uint32_t slot = (n % kSlots) * kSlotBytes;
 #pragma unroll
         for (int ks = 0; ks < kDo / 16; ++ks)
-          umma_bf16_ts(tmem + kColS, tmem + kColQ + ks * 8, umma_desc_k_sw128(kv + (ks >> 2) * kSubBytes + (ks & 3) * 32), id_qk, ks != 0);
+          umma_bf16_ts(td + kColS, td + kColQ + ks * 8, d_lat + ((slot + (ks >> 2) * kSubBytes + (ks & 3) * 32) >> 4), id_qk, ks != 0, issue);
 #pragma unroll
         for (int ks = 0; ks < kDr / 32; ++ks)
-          umma_bf16_ts(tmem + kColS, tmem + kColQ + kDo / 2 + ks * 8, umma_desc_k_sw64(kv + kLatBytes + ks * 32), id_qk, true);
-        umma_commit(&s_full);
+          umma_bf16_ts(td + kColS, td + kColQ + kDo / 2 + ks * 8, d_rope + ((slot + ks * 32) >> 4), id_qk, 1u, issue);
+        umma_commit_by(&s_full[n & 1], issue);
         return true;
       };
+      uint32_t n_seg = 0;
       while (ok && walk.next(s_seq, p, seg)) {
-        ok = mbar_wait(&q_full, n_seg & 1, deadline);
+        ok = wait(&q_full, n_seg & 1);
         ++n_seg;
         if (ok) {
           tc_fence_after_sync();
@@ -590,22 +669,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             ok = false;
             break;
           }
-          if (!mbar_wait(&p_full, n & 1, deadline)) {
+          if (!wait(&p_full, n & 1)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint32_t kv = smem_u32(smem) + (n % kSlots) * kSlotBytes;
+          const uint32_t slot = (n % kSlots) * kSlotBytes;
 #pragma unroll
           for (int ks = 0; ks < kTile / 16; ++ks)
-            umma_bf16_ts(tmem + kColO, tmem + kColP + ks * 8, umma_desc_mn_sw128(kv + ks * 2048, kSubBytes), id_pv, i != 0 || ks != 0);
-          umma_commit(&kv_free[n % kSlots]);
+            umma_bf16_ts(td + kColO, td + kColP + ks * 8, d_val + ((slot + ks * 2048) >> 4), id_pv, (i | ks) != 0, issue);
+          umma_commit_by(&kv_free[n % kSlots], issue);
         }
         gt += seg.count;
       }
       if (!ok) {
-        atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
-        umma_commit(&drain);                           // nothing of this CTA's may be in flight when it leaves
+        if (lane == 0) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
+        umma_commit_by(&drain, issue);                 // nothing of this CTA's may be in flight when it leaves
         mbar_wait(&drain, 0, now_ns() + 10000000ull);
       }
     }
@@ -622,15 +701,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_arrive();
   cluster_wait();
   tc_fence_after_sync();
-  if (warp == kSmWarps + kDqWarps) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // Merges the pieces of every sequence that more than one cluster worked on, and writes the empty sequences' zeros.
-// Block (b, y) takes `heads` heads of sequence b, thread t output columns [4 t, 4 t + 4).
-__global__ void __launch_bounds__(kDn / 4) mla_pair_fold_kernel(const __grid_constant__ MlaDecodeParams p, int n_clusters, int heads) {
+// Block (b, y) takes `heads` heads of sequence b.  Threads come in groups of 128 that share out the pieces, thread t of a
+// group has output columns [4 t, 4 t + 4); with few sequences there are few blocks and many pieces each, so more groups.
+constexpr int kFoldCols = kDn / 4, kFoldMaxGroups = 4;
+__global__ void __launch_bounds__(kFoldCols * kFoldMaxGroups)
+    mla_pair_fold_kernel(const __grid_constant__ MlaDecodeParams p, int n_clusters, int heads) {
   __shared__ int s_sum[2];
-  __shared__ float s_w[kDn / 4], s_red[4];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = blockIdx.x;
+  __shared__ float s_w[kMlaMaxCtas / 2], s_l;
+  __shared__ float4 s_acc[kFoldMaxGroups - 1][kFoldCols];
+  const int tid = threadIdx.x, lane = tid & 31, b = blockIdx.x;
+  const int t = tid % kFoldCols, g = tid / kFoldCols, groups = blockDim.x / kFoldCols;
   if (tid < 2) s_sum[tid] = 0;
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -646,50 +730,64 @@ __global__ void __launch_bounds__(kDn / 4) mla_pair_fold_kernel(const __grid_con
   const int n_tiles = max((p.seq_lens[b] + kTile - 1) / kTile, 0);
   __syncthreads();
   const int base = s_sum[0], chunk = max((s_sum[1] + n_clusters - 1) / n_clusters, 1);
-  const int first = base / chunk, last = (base + max(n_tiles, 1) - 1) / chunk;
-  if (n_tiles > 0 && first == last) return;
+  const int first = base / chunk, last = (base + max(n_tiles, 1) - 1) / chunk, n = last - first + 1;
+  if (n_tiles > 0 && n == 1) return;
   for (int h = blockIdx.y * heads; h < min((int)(blockIdx.y + 1) * heads, kH); ++h) {
-    uint2* dst = reinterpret_cast<uint2*>(p.o + ((int64_t)b * kH + h) * kDn) + tid;
+    uint2* dst = reinterpret_cast<uint2*>(p.o + ((int64_t)b * kH + h) * kDn) + t;
     if (n_tiles == 0) {
-      *dst = make_uint2(0u, 0u);
+      if (g == 0) *dst = make_uint2(0u, 0u);
       if (tid == 0) p.lse[(int64_t)b * kH + h] = -INFINITY;
       continue;
     }
     // the first piece starts its sequence (slot 1); every later one begins where its cluster begins (slot 0)
-    auto slot = [&](int c) { return (size_t)c * 2 + (c == first ? 1 : 0); };
-    float M = -INFINITY;
-    for (int c = first + lane; c <= last; c += 32) M = fmaxf(M, __ldcg(p.part_lse + slot(c) * kH + h));
+    auto slot = [&](int i) { return (size_t)(first + i) * 2 + (i == 0 ? 1 : 0); };
+    if (tid < 32) {
+      float M = -INFINITY, L = 0.f;
+      for (int i = lane; i < n; i += 32) {
+        const float l = __ldcg(p.part_lse + slot(i) * kH + h);
+        s_w[i] = l;
+        M = fmaxf(M, l);
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float L = 0.f;
-    for (int c0 = first; c0 <= last; c0 += kDn / 4) {
-      const int nb = min(kDn / 4, last - c0 + 1);
-      __syncthreads();
-      float w = 0.f;
-      if (tid < nb && M != -INFINITY) w = fast_exp2(__ldcg(p.part_lse + slot(c0 + tid) * kH + h) - M);
-      s_w[tid] = w;
+      for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+      for (int i = lane; i < n; i += 32) {
+        const float w = M == -INFINITY ? 0.f : fast_exp2(s_w[i] - M);
+        s_w[i] = w;
+        L += w;
+      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-      if (lane == 0) s_red[warp] = w;
-      __syncthreads();
-      L += s_red[0] + s_red[1] + s_red[2] + s_red[3];
-#pragma unroll 8
-      for (int j = 0; j < nb; ++j) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.part_o + (slot(c0 + j) * kH + h) * kDn) + tid);
-        const float wj = s_w[j];
-        acc.x += wj * v.x;
-        acc.y += wj * v.y;
-        acc.z += wj * v.z;
-        acc.w += wj * v.w;
+      for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+      if (lane == 0) {
+        s_l = L;
+        const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
+        p.lse[(int64_t)b * kH + h] = p.lse_base2 ? lse2 : lse2 * kLn2;
       }
     }
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    *dst = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
-    if (tid == 0) {
-      const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
-      p.lse[(int64_t)b * kH + h] = p.lse_base2 ? lse2 : lse2 * kLn2;
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int i = g; i < n; i += groups) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p.part_o + (slot(i) * kH + h) * kDn) + t);
+      const float w = s_w[i];
+      acc.x += w * v.x;
+      acc.y += w * v.y;
+      acc.z += w * v.z;
+      acc.w += w * v.w;
     }
+    if (g > 0) s_acc[g - 1][t] = acc;
+    __syncthreads();
+    if (g == 0) {
+      for (int k = 1; k < groups; ++k) {
+        const float4 v = s_acc[k - 1][t];
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+      }
+      const float inv = s_l > 0.f ? 1.f / s_l : 0.f;
+      *dst = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+    }
+    __syncthreads();                            // s_w, s_l and s_acc are free again
   }
 }
 
@@ -718,9 +816,11 @@ cudaError_t launch_mla_decode_pair(const MlaDecodeParams& p, bool pdl, cudaStrea
   e = cudaLaunchKernelEx(&cfg, mla_pair_kernel, p);
   if (e != cudaSuccess) return e;
   // The fold is always chained to this launch: it waits for the whole grid before it reads anything.
-  const int heads = p.B >= 16 ? 8 : p.B >= 4 ? 2 : 1;
+  // A block's heads follow one another, 2-3 us each, so it takes several only where one each would be more blocks than
+  // the device holds at once (16 of them per SM).
+  const int heads = p.B <= 18 ? 1 : p.B <= 37 ? 2 : 4;
   cfg.gridDim = dim3(p.B, kH / heads, 1);
-  cfg.blockDim = dim3(kDn / 4, 1, 1);
+  cfg.blockDim = dim3(kFoldCols * (p.B <= 4 ? 4 : p.B <= 9 ? 2 : 1), 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, mla_pair_fold_kernel, p, p.ctas / 2, heads);

@@ -53,10 +53,11 @@ def _check(seq_lens, page, ctas, scale, base2=False, std=0.5, poison=False):
 
 
 # edges of the 64-token tile and of the 16-token unit, one to several tiles a piece, more sequences than clusters, empty
-# sequences, pieces whose boundaries fall inside and between sequences
+# sequences, pieces whose boundaries fall inside and between sequences, every shape of the fold (by batch size)
 @pytest.mark.parametrize("seq_lens,page,ctas", [
     ([1], 16, 0), ([64], 16, 0), ([15, 16, 17, 63, 64, 65], 16, 2), ([127, 0, 128, 129], 32, 4), ([300, 1, 700], 48, 6),
-    ([1024], 64, 2), ([1000], 64, 32), ([5, 0, 64] * 70, 16, 0), ([2049, 640, 4096], 32, 10), ([20000], 16, 0)])
+    ([1024], 64, 2), ([1000], 64, 32), ([5, 0, 64] * 70, 16, 0), ([2049, 640, 4096], 32, 10), ([20000], 16, 0),
+    ([2000] * 6, 16, 0), ([300, 900] * 10, 32, 0), ([700] * 40, 16, 0)])
 def test_pair_kernel_matches_fp32_reference(native_built, seq_lens, page, ctas):
     _check(seq_lens, page, ctas, 1.0 / math.sqrt(192))
 
