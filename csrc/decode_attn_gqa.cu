@@ -667,8 +667,9 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
 constexpr int kFoldThreads = 128;
 __global__ void __launch_bounds__(kFoldThreads) gqa_fold_kernel(const __grid_constant__ GqaDecodeParams p) {
   __shared__ unsigned short s_list[kMaxList];
-  __shared__ float4 s_acc[kFoldThreads / 32 - 1][32];
-  __shared__ float s_red[kFoldThreads / 32];
+  __shared__ float4 s_acc[kFoldThreads / 32][32];
+  __shared__ float s_max[kFoldThreads / 32], s_sum[kFoldThreads / 32];
+  static_assert(kFoldThreads == 128, "four warps");
   __shared__ int s_n;
   __shared__ long long s_part[2];
   __shared__ int s_nb[kGqaSeqTable];
@@ -703,41 +704,61 @@ __global__ void __launch_bounds__(kFoldThreads) gqa_fold_kernel(const __grid_con
     }
   }
   for (int hg = blockIdx.y; hg < group; hg += gridDim.y) {
-    // weights of the pieces
-    float M = -INFINITY;
-    for (int i = tid; i < n; i += kFoldThreads) M = fmaxf(M, __ldcg(p.part_lse + (size_t)s_list[i] * 8 + hg));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    if (lane == 0) s_red[warp] = M;
-    __syncthreads();
-    M = s_red[0];
-#pragma unroll
-    for (int w = 1; w < kFoldThreads / 32; ++w) M = fmaxf(M, s_red[w]);
-    float L = 0.f;
+    // Each warp takes every fourth piece, eight rows and their LSEs per round trip, with a running maximum of its own
+    // (one round trip less than weights first: 1 x 32768 tokens 35.4 -> 34.3 us, 1 x 131072 90.8 -> 89.9; batches with few
+    // pieces per pair are level, within 1 %).
+    float M = -INFINITY, L = 0.f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int i = warp; i < n; i += kFoldThreads / 32) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(p.part_o + ((size_t)s_list[i] * 8 + hg) * kD) + lane);
-      const float l = __ldcg(p.part_lse + (size_t)s_list[i] * 8 + hg), w = l == -INFINITY ? 0.f : fast_exp2(l - M);
-      L += w;
-      acc.x += w * v.x;
-      acc.y += w * v.y;
-      acc.z += w * v.z;
-      acc.w += w * v.w;
+    for (int i0 = warp; i0 < n; i0 += 8 * (kFoldThreads / 32)) {
+      float4 v[8];
+      float l[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * (kFoldThreads / 32);
+        l[j] = -INFINITY;
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n) {
+          const size_t row = (size_t)s_list[i] * 8 + hg;
+          l[j] = __ldcg(p.part_lse + row);
+          v[j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + row * kD) + lane);
+        }
+      }
+      float top = M;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) top = fmaxf(top, l[j]);
+      const float keep = M == -INFINITY ? 0.f : fast_exp2(M - top);
+      M = top;
+      L *= keep;
+      acc = make_float4(acc.x * keep, acc.y * keep, acc.z * keep, acc.w * keep);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float w = l[j] == -INFINITY ? 0.f : fast_exp2(l[j] - top);
+        L += w;
+        acc.x += w * v[j].x;
+        acc.y += w * v[j].y;
+        acc.z += w * v[j].z;
+        acc.w += w * v[j].w;
+      }
     }
-    __syncthreads();                            // s_red is read
-    if (warp > 0) s_acc[warp - 1][lane] = acc;
-    if (lane == 0) s_red[warp] = L;
+    s_acc[warp][lane] = acc;
+    if (lane == 0) {
+      s_max[warp] = M;
+      s_sum[warp] = L;
+    }
     __syncthreads();
     if (warp == 0) {
+      M = fmaxf(fmaxf(s_max[0], s_max[1]), fmaxf(s_max[2], s_max[3]));
+      L = 0.f;
+      acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int w = 1; w < kFoldThreads / 32; ++w) {
-        const float4 v = s_acc[w - 1][lane];
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-        L += s_red[w];
+      for (int w = 0; w < kFoldThreads / 32; ++w) {
+        const float f = s_max[w] == -INFINITY ? 0.f : fast_exp2(s_max[w] - M);
+        const float4 v = s_acc[w][lane];
+        L += f * s_sum[w];
+        acc.x += f * v.x;
+        acc.y += f * v.y;
+        acc.z += f * v.z;
+        acc.w += f * v.w;
       }
       const float inv = L > 0.f ? 1.f / L : 0.f;
       const int64_t row = (int64_t)b * p.Hq + kvh * group + hg;
@@ -747,7 +768,7 @@ __global__ void __launch_bounds__(kFoldThreads) gqa_fold_kernel(const __grid_con
         p.lse[row] = p.lse_base2 ? lse2 : lse2 * kLn2;
       }
     }
-    __syncthreads();                            // s_acc and s_red are free again
+    __syncthreads();                            // s_acc, s_max and s_sum are free again
   }
 }
 
