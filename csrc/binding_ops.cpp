@@ -226,8 +226,10 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   // HELIX_A2A_MLA_VARIANT: "pair" = clusters of two CTAs, "ws" = producer warps + math warps, "lockstep" = all warps in
   // lockstep
   const char* v = std::getenv("HELIX_A2A_MLA_VARIANT");
-  const int variant = !v ? kMlaDefaultVariant
-                         : std::string(v) == "lockstep" ? 0 : std::string(v) == "ws" ? 1 : kMlaDefaultVariant;
+  int variant = !v ? kMlaDefaultVariant
+                   : std::string(v) == "lockstep" ? 0 : std::string(v) == "ws" ? 1 : kMlaDefaultVariant;
+  // the pair kernel reads q_nope 16 bytes at a time, the others 4: a view with an odd storage offset stays with those
+  if (variant == 2 && reinterpret_cast<uintptr_t>(q_nope.data_ptr()) % 16 != 0) variant = 1;
   const int longest = (int)std::max<int64_t>(max_seq_len, 1);
   int nc = ctas > 0 ? (int)std::min<int64_t>(ctas, helix::kMlaMaxCtas)
            : variant == 2 ? helix::mla_pair_pick_ctas(B, longest, helix::device_sm_count())

@@ -83,3 +83,14 @@ def test_pair_kernel_rescales_and_agrees_with_one_piece(native_built):
         assert (lse - l_ref).abs().max() < 5e-2
         # scores here are off by up to 0.25 * 0.5 * 2^-8 * sqrt(512) = 0.011, so weights by 1.1 %
         assert (o.float() - o_ref).abs().max() < 0.1
+
+
+def test_unaligned_queries_keep_a_kernel_that_takes_them(native_built):
+    """A contiguous q_nope that starts 4 bytes off a 16-byte boundary (a view into a larger buffer)."""
+    from helix_a2a_b200.ops import attention
+    qn, qp, ckv, scales, kpe, bt, sl = _case([200, 33], 16, seed=9)
+    shifted = torch.empty(qn.numel() + 8, dtype=qn.dtype, device="cuda")[2:2 + qn.numel()].view_as(qn).copy_(qn)
+    assert shifted.data_ptr() % 16 == 4 and shifted.is_contiguous()
+    want, got = (attention.mla_decode(q, qp, ckv, scales, kpe, bt, sl, scale=0.07, max_seq_len=200) for q in (qn, shifted))
+    # two kernels of the same precision: one bf16 rounding of values up to about 4.5 apart, and of the probabilities
+    assert (want[0].float() - got[0].float()).abs().max() < 3e-2 and (want[1] - got[1]).abs().max() < 1e-3
