@@ -22,12 +22,13 @@
 // the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19 dequantise, fed by register prefetch two tiles ahead.  The MMA queue
 // runs Q K^T two tiles ahead of P V.
 // Pieces of a sequence are merged by a second small kernel (mla_pair_fold_kernel) with all SMs.
-// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 662 -> 445 us, 16 ragged
-// sequences up to 17000 tokens 253 -> 88 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
-// On the way there: one softmax group whose threads exchanged all partial scores, 606 us with buffer credits and 495
-// without; two groups 478; each CTA finishing half of the heads 445.  A third of the warps more (32 tokens a thread)
-// lost: 520.  A tile takes about 3000 cycles, of which the tensor pipe is busy 2100: an MMA with A in tensor memory and
-// N = 64 takes 83 cycles (32 of them arithmetic), P V's with N = 256 170.
+// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 430 us, 16 ragged
+// sequences up to 17000 tokens 251 -> 86 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
+// On the way there (32 x 32768): one softmax group whose threads exchanged all partial scores, 606 us with buffer
+// credits and 495 without; two groups 478; each CTA finishing half of the heads 445; MMAs issued under one convergent
+// elect with operands in uniform registers 430.  Lost: a third of the warps more (32 tokens a thread, 520); a second score
+// buffer with a quarter of Q in shared memory (446 against 445); a tile exchanged in two halves (461 against 445); the
+// next scores fetched before P goes out (573 against 393 in a graph: the registers spill).
 // Every wait is bounded; on expiry the error flag is raised, tensor memory is released and the kernel returns.
 #include "attention.h"
 
@@ -120,25 +121,31 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&v)[
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem desc], A with two bf16 of the K index per 32-bit column; the whole warp comes here and
-// the lane with `issue` set issues
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate,
-                                             uint32_t issue) {
+// D[tmem] (+)= A[tmem] * B[smem desc], A with two bf16 of the K index per 32-bit column; issued by one lane.  The
+// descriptor comes as two words: only the lower one, with the address, differs between calls.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi, uint32_t idesc) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
+      "{\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, 1;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit_by(uint64_t* bar, uint32_t issue) {
+__device__ __forceinline__ void umma_bf16_ts_first(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi, uint32_t idesc,
+                                                   uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(smem_u32(bar)), "r"(issue)
+      "{\n\t.reg .b64 d;\n\t.reg .pred p;\n\t"
+      "mov.b64 d, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// one lane of a warp that has come here together, always the same
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
 }
 // K-major operand of 64-byte rows with the 64-byte swizzle, 8-row groups 512 bytes apart
 __device__ __forceinline__ uint64_t umma_desc_k_sw64(uint32_t addr) {
@@ -633,25 +640,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (warp == 0) {
       constexpr uint32_t id_qk = umma_idesc_bf16(kH, kTile);
       constexpr uint32_t id_pv = umma_idesc_bf16(kH, kDo) | (1u << 16);       // B is MN-major
-      const uint32_t issue = lane == 0 ? 1u : 0u;
-      const uint32_t td = __shfl_sync(0xffffffffu, tmem, 0);
+      // All 512 columns are this CTA's, so its tensor memory starts at column 0: no register holds the base.  The tile
+      // number goes through a shuffle for the same reason: what is computed from it is then known to be the same in all lanes
+      // and stays in uniform registers, which is where the MMA reads its operands (moving them there cost ~60 cycles each).
+      constexpr uint32_t td = 0;
       const uint64_t d_lat = umma_desc_k_sw128(smem_u32(smem)), d_rope = umma_desc_k_sw64(smem_u32(smem) + kLatBytes),
                      d_val = umma_desc_mn_sw128(smem_u32(smem), kSubBytes);
       // every lane waits, so that the warp stays together and all agree
       auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, deadline)) != 0; };
       // byte offsets enter a descriptor in 16-byte units and never carry out of its 14-bit address field
-      auto qk = [&](uint32_t n) {
+      auto qk = [&](uint32_t n_lane) {
+        const uint32_t n = __shfl_sync(0xffffffffu, n_lane, 0);
         if (!wait(&kv_full[n % kSlots], (n / kSlots) & 1)) return false;
         if (n >= 1 && !wait(&s_free, (n - 1) & 1)) return false;
         tc_fence_after_sync();
         const uint32_t slot = (n % kSlots) * kSlotBytes;
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kDo / 16; ++ks)
-          umma_bf16_ts(td + kColS, td + kColQ + ks * 8, d_lat + ((slot + (ks >> 2) * kSubBytes + (ks & 3) * 32) >> 4), id_qk, ks != 0, issue);
+          for (int ks = 0; ks < kDo / 16; ++ks) {
+            const uint32_t lo = (uint32_t)d_lat + ((slot + (ks >> 2) * kSubBytes + (ks & 3) * 32) >> 4);
+            if (ks == 0) umma_bf16_ts_first(td + kColS, td + kColQ, lo, (uint32_t)(d_lat >> 32), id_qk, 0u);
+            else umma_bf16_ts(td + kColS, td + kColQ + ks * 8, lo, (uint32_t)(d_lat >> 32), id_qk);
+          }
 #pragma unroll
-        for (int ks = 0; ks < kDr / 32; ++ks)
-          umma_bf16_ts(td + kColS, td + kColQ + kDo / 2 + ks * 8, d_rope + ((slot + ks * 32) >> 4), id_qk, 1u, issue);
-        umma_commit_by(&s_full[n & 1], issue);
+          for (int ks = 0; ks < kDr / 32; ++ks)
+            umma_bf16_ts(td + kColS, td + kColQ + kDo / 2 + ks * 8, (uint32_t)d_rope + ((slot + ks * 32) >> 4), (uint32_t)(d_rope >> 32), id_qk);
+          umma_commit(&s_full[n & 1]);
+        }
+        __syncwarp();
         return true;
       };
       uint32_t n_seg = 0;
@@ -664,7 +680,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         if (ok && seg.count > 1) ok = qk(gt + 1);
         for (int i = 0; i < seg.count && ok; ++i) {
-          const uint32_t n = gt + i;
+          const uint32_t n = __shfl_sync(0xffffffffu, gt + i, 0), later = __shfl_sync(0xffffffffu, i, 0);
           if (i + 2 < seg.count && !qk(n + 2)) {
             ok = false;
             break;
@@ -675,16 +691,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
           tc_fence_after_sync();
           const uint32_t slot = (n % kSlots) * kSlotBytes;
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < kTile / 16; ++ks)
-            umma_bf16_ts(td + kColO, td + kColP + ks * 8, d_val + ((slot + ks * 2048) >> 4), id_pv, (i | ks) != 0, issue);
-          umma_commit_by(&kv_free[n % kSlots], issue);
+            for (int ks = 0; ks < kTile / 16; ++ks) {
+              const uint32_t lo = (uint32_t)d_val + ((slot + ks * 2048) >> 4);
+              if (ks == 0) umma_bf16_ts_first(td + kColO, td + kColP, lo, (uint32_t)(d_val >> 32), id_pv, later);
+              else umma_bf16_ts(td + kColO, td + kColP + ks * 8, lo, (uint32_t)(d_val >> 32), id_pv);
+            }
+            umma_commit(&kv_free[n % kSlots]);
+          }
+          __syncwarp();
         }
         gt += seg.count;
       }
       if (!ok) {
         if (lane == 0) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
-        umma_commit_by(&drain, issue);                 // nothing of this CTA's may be in flight when it leaves
+        if (elect_one()) umma_commit(&drain);                 // nothing of this CTA's may be in flight when it leaves
         mbar_wait(&drain, 0, now_ns() + 10000000ull);
       }
     }
