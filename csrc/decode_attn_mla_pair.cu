@@ -19,8 +19,8 @@
 // Roles per CTA (20 warps): warp 0 issues the MMAs (the oldest warp, so that busier ones do not keep it waiting; the
 // whole warp walks the loop and one lane issues, which lets the operands stay in uniform registers); warps 4..7 and 8..11
 // are two groups that take tiles in turn (thread = one head; two warps of a group finish this CTA's heads, two forward
-// the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19 dequantise, fed by register prefetch two tiles ahead.  The MMA queue
-// runs Q K^T two tiles ahead of P V.
+// the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19
+// dequantise, fed by register prefetch two tiles ahead.  The MMA queue runs Q K^T two tiles ahead of P V.
 // Pieces of a sequence are merged by a second small kernel (mla_pair_fold_kernel) with all SMs.
 // Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 430 us, 16 ragged
 // sequences up to 17000 tokens 251 -> 86 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
