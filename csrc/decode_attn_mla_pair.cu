@@ -20,13 +20,14 @@
 // whole warp walks the loop and one lane issues, which lets the operands stay in uniform registers); warps 4..7 and 8..11
 // are two groups that take tiles in turn (thread = one head; two warps of a group finish this CTA's heads, two forward
 // the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19
-// dequantise, fed by register prefetch two tiles ahead.  The MMA queue runs Q K^T two tiles ahead of P V.
+// dequantise, fed by register prefetch one tile ahead.  The MMA queue runs Q K^T two tiles ahead of P V.
 // Pieces of a sequence are merged by a second small kernel (mla_pair_fold_kernel) with all SMs.
-// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 430 us, 16 ragged
-// sequences up to 17000 tokens 251 -> 86 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 27 us.
+// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 419 us, 16 ragged
+// sequences up to 17000 tokens 252 -> 84 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 26 us.
 // On the way there (32 x 32768): one softmax group whose threads exchanged all partial scores, 606 us with buffer
 // credits and 495 without; two groups 478; each CTA finishing half of the heads 445; MMAs issued under one convergent
-// elect with operands in uniform registers 430.  Lost: a third of the warps more (32 tokens a thread, 520); a second score
+// elect with operands in uniform registers 430; one tile of prefetch instead of two, whose registers the softmax warps
+// put to better use, 419.  Lost: a third of the warps more (32 tokens a thread, 520); a second score
 // buffer with a quarter of Q in shared memory (446 against 445); a tile exchanged in two halves (461 against 445); the
 // next scores fetched before P goes out (573 against 393 in a graph: the registers spill).
 // Every wait is bounded; on expiry the error flag is raised, tensor memory is released and the kernel returns.
@@ -311,7 +312,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
   if (warp >= kFirstSm && warp < kFirstDq) {
     // =========================== softmax ===========================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
     const int quad = warp & 3, h = 32 * quad + lane;
     const uint32_t grp = (uint32_t)(warp - kFirstSm) / kGroupWarps;     // this group takes tiles n with n % 2 == grp
     const uint32_t tq = tmem + ((uint32_t)(32 * quad) << 16);           // this warp's lanes of the tensor memory
@@ -537,7 +538,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (!ok && lane == 0) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
   } else if (warp >= kFirstDq) {
     // =========================== dequantisation ===========================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     const int w8 = warp - kFirstDq;
     // Eight consecutive lanes (one phase of a 16-byte shared-memory access) hold four chunks of an even row and the
     // four of the odd row below: their swizzled stores fall in all eight 16-byte bank groups.
@@ -619,19 +620,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       if (lane == 0) mbar_arrive(&kv_full[gt % kSlots]);
       ++gt;
     };
-    Fetch fa, fb;
+    Fetch f;
     advance();
-    load(fa);
-    load(fb);
-    while (true) {
-      if (fa.live == 0) break;
-      convert(fa);
+    load(f);
+    while (f.live != 0) {
+      convert(f);
       if (!ok) break;
-      load(fa);
-      if (fb.live == 0) break;
-      convert(fb);
-      if (!ok) break;
-      load(fb);
+      load(f);
     }
     if (!ok) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
   } else {
