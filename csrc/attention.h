@@ -31,8 +31,9 @@ struct GqaDecodeParams {
   //   [2P + 8, ...)   one flag per helper slot: a piece has been parked there
   int* counters;
   int* error_flag;             // set to a helix::Status code when a bounded wait runs out
-  unsigned long long* trace;   // optional [ctas][8] stamps (%globaltimer): entry, first data, end of the fixed share,
+  unsigned long long* trace;   // optional [gqa_grid][8] stamps (%globaltimer): entry, first data, end of the fixed share,
                                // exit, end of the last drawn chunk, chunks drawn | pools visited << 32, SM id
+  int trace_rows;              // rows `trace` has room for: a launch with more CTAs is refused
   int B, Hq, Hkv, page_size, ctas;
   int whole;                   // 1: one CTA per (sequence, kv head) pair (grid B * Hkv, `ctas` unused), nothing is split
   // Dynamic tail: of every pair with at least dyn_min_blocks KV blocks, the last dyn_pct percent (rounded down to
@@ -49,7 +50,7 @@ struct GqaDecodeParams {
   unsigned long long timeout_ns;
 };
 
-constexpr int kGqaMaxCtas = 640;     // upper bound of the grid
+constexpr int kGqaMaxCtas = 640;     // upper bound of the grid when pairs are split
 constexpr int kGqaMaxHelper = 1024;  // upper bound of the chunks all dynamic pools hold together
 constexpr int kGqaSeqTable = 256;    // batches beyond this run with fixed shares only
 
@@ -57,6 +58,9 @@ constexpr int kGqaSeqTable = 256;    // batches beyond this run with fixed share
 constexpr size_t gqa_part_o_floats(int ctas, int max_helper) { return ((size_t)ctas * 2 + max_helper) * 8 * 128; }
 constexpr size_t gqa_part_lse_floats(int ctas, int max_helper) { return ((size_t)ctas * 2 + max_helper) * 8; }
 constexpr size_t gqa_counter_ints(int pairs, int max_helper) { return (size_t)2 * pairs + 8 + max_helper; }
+
+// CTAs of the streaming launch: at most kGqaMaxCtas when pairs are split, but as many as there are pairs when they are whole
+inline int gqa_grid(const GqaDecodeParams& p) { return p.whole ? p.B * p.Hkv : p.ctas; }
 
 // number of CTAs that fills the device for this batch (two per SM unless the work is tiny)
 int gqa_pick_ctas(int B, int Hkv, int max_seq_len, int sm_count);

@@ -36,7 +36,7 @@ struct Scratch {
   torch::Tensor error_flag;    // int32 [1]
   torch::Tensor counters;      // int32 [N]
   torch::Tensor part_a, part_b;  // float32 pools
-  torch::Tensor trace;           // int64 [kGqaMaxCtas * 8], only with HELIX_A2A_ATTN_TRACE=1 / HELIX_A2A_OPROJ_TRACE=1
+  torch::Tensor trace;           // int64 [rows * 8], only with one of the *_TRACE / *_PROF variables set
   std::vector<torch::Tensor> retired;
 };
 std::mutex g_mu;
@@ -58,6 +58,15 @@ Scratch& scratch_for(const torch::Device& dev, int64_t counters, int64_t part_a_
   grow(s.part_a, part_a_floats, 1, fopt, false);
   grow(s.part_b, part_b_floats, 1, fopt, false);
   return s;
+}
+
+// Eight int64 stamps for each of `rows` CTAs.  A tensor that has become too small is kept like the other buffers.
+unsigned long long* trace_for(Scratch& s, const torch::Device& dev, int64_t rows) {
+  if (!s.trace.defined() || s.trace.numel() < rows * 8) {
+    if (s.trace.defined()) s.retired.push_back(s.trace);
+    s.trace = torch::zeros({std::max<int64_t>(rows, helix::kGqaMaxCtas) * 8}, torch::TensorOptions().dtype(torch::kInt64).device(dev));
+  }
+  return reinterpret_cast<unsigned long long*>(s.trace.data_ptr());
 }
 
 int env_int(const char* name, int dflt) {
@@ -181,8 +190,8 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   {
     const char* tr = std::getenv("HELIX_A2A_ATTN_TRACE");
     if (tr && tr[0] == '1') {
-      if (!sc.trace.defined()) sc.trace = torch::zeros({helix::kGqaMaxCtas * 8}, q.options().dtype(torch::kInt64));
-      p.trace = reinterpret_cast<unsigned long long*>(sc.trace.data_ptr());
+      p.trace_rows = helix::gqa_grid(p);
+      p.trace = trace_for(sc, q.device(), p.trace_rows);
     }
   }
   p.kv_stable = kv_stable ? 1 : 0;
@@ -260,10 +269,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   p.prof = nullptr;
   {
     static const bool prof_on = [] { const char* v = std::getenv("HELIX_A2A_MLA_PROF"); return v && std::string(v) == "1"; }();
-    if (prof_on) {
-      if (!sc.trace.defined()) sc.trace = torch::zeros({helix::kGqaMaxCtas * 8}, q_nope.options().dtype(torch::kInt64));
-      p.prof = reinterpret_cast<unsigned long long*>(sc.trace.data_ptr());
-    }
+    if (prof_on) p.prof = trace_for(sc, q_nope.device(), nc);
   }
   check_cuda(helix::launch_mla_decode(p, env_pdl(), stream), "mla decode launch");
   return std::make_tuple(o, lse);
@@ -321,10 +327,7 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     p.trace = nullptr;
     if (streamk) {
       static const bool trace_on = [] { const char* v = std::getenv("HELIX_A2A_OPROJ_TRACE"); return v && std::string(v) == "1"; }();
-      if (trace_on) {
-        if (!sc.trace.defined()) sc.trace = torch::zeros({helix::kGqaMaxCtas * 8}, x.options().dtype(torch::kInt64));
-        p.trace = reinterpret_cast<unsigned long long*>(sc.trace.data_ptr());
-      }
+      if (trace_on) p.trace = trace_for(sc, x.device(), sk_ctas);
     }
     check_cuda(streamk          ? helix::launch_oproj_streamk(p, env_pdl(), stream)
                : plan.slabs > 0 ? helix::launch_oproj_split(p, plan.slabs, env_pdl(), stream)
@@ -445,10 +448,7 @@ std::tuple<torch::Tensor, torch::Tensor> fused_impl(torch::Tensor attn_out, torc
   {
     // per-CTA %globaltimer stamps of the one-kernel path (read back with attn_trace)
     static const bool trace_on = [] { const char* v = std::getenv("HELIX_A2A_EXCHANGE_TRACE"); return v && std::string(v) == "1"; }();
-    if (trace_on) {
-      if (!sc.trace.defined()) sc.trace = torch::zeros({helix::kGqaMaxCtas * 8}, attn_out.options().dtype(torch::kInt64));
-      p.trace = reinterpret_cast<unsigned long long*>(sc.trace.data_ptr());
-    }
+    if (trace_on) p.trace = trace_for(sc, attn_out.device(), helix::kGqaMaxCtas);
   }
   for (int r = 0; r < ranks; ++r) {
     p.io[r].o_src = reinterpret_cast<const uint8_t*>(attn_out.data_ptr()) + (int64_t)r * B * H * D * 2;

@@ -815,7 +815,8 @@ void gqa_plan_dynamic(GqaDecodeParams* p, int max_seq_len, int max_helper, int p
 cudaError_t launch_gqa_decode(const GqaDecodeParams& p, bool pdl, cudaStream_t stream) {
   if (p.B <= 0) return cudaSuccess;
   if (p.Hq % p.Hkv != 0 || p.Hq / p.Hkv > 8 || p.page_size % kBlockTok != 0 || p.ctas < 1 || p.ctas > kGqaMaxCtas ||
-      p.max_helper < 0 || p.max_helper > kGqaMaxHelper || p.dyn_pct < 0 || p.dyn_pct > 50)
+      p.max_helper < 0 || p.max_helper > kGqaMaxHelper || p.dyn_pct < 0 || p.dyn_pct > 50 ||
+      (p.trace != nullptr && gqa_grid(p) > p.trace_rows))
     return cudaErrorInvalidValue;
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -828,7 +829,7 @@ cudaError_t launch_gqa_decode(const GqaDecodeParams& p, bool pdl, cudaStream_t s
     if (dev < 64) attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.whole ? p.B * p.Hkv : p.ctas, 1, 1);
+  cfg.gridDim = dim3(gqa_grid(p), 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;

@@ -40,3 +40,20 @@ def test_forms_agree_with_the_oracle(native_built, lens, hkv, group, page, layou
         assert (o.cpu().float() - o_ref.float()).abs().max() < 2e-2, splits
         assert (lse.cpu()[live] - l_ref[live]).abs().max() < 1e-3, splits
         assert torch.isneginf(lse.cpu()[~live]).all()
+
+
+# 1024 unsplit pairs are more CTAs than any split launch has; 2 x 20000 tokens are split
+@pytest.mark.parametrize("lens,hkv", [([40, 17, 0, 300] * 32, 8), ([20000, 700], 8)])
+def test_time_stamps_have_a_row_for_every_cta(native_built, monkeypatch, lens, hkv):
+    from helix_a2a_b200.ops import attention
+    from helix_a2a_b200.ops._ext import ext, ops
+    q, k, v, bt, sl = _case(lens, hkv, 8, 16, "HND", 5)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ctas = len(lens) * hkv if max(lens) < 1000 else ext().gqa_pick_ctas(len(lens), hkv, max(lens), sms)
+    monkeypatch.setenv("HELIX_A2A_ATTN_DYN_PCT", "0")            # fixed shares: who streams what does not change from call to call
+    want = attention.gqa_decode(q, k, v, bt, sl, max_seq_len=max(lens))
+    monkeypatch.setenv("HELIX_A2A_ATTN_TRACE", "1")
+    got = attention.gqa_decode(q, k, v, bt, sl, max_seq_len=max(lens))
+    stamps = ops().attn_trace(q).view(-1, 8)
+    assert stamps.shape[0] >= ctas and (stamps[:ctas, 3] >= stamps[:ctas, 0]).all() and (stamps[:ctas, 0] > 0).all()
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
