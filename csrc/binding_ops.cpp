@@ -237,8 +237,15 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   const char* v = std::getenv("HELIX_A2A_MLA_VARIANT");
   int variant = !v ? kMlaDefaultVariant
                    : std::string(v) == "lockstep" ? 0 : std::string(v) == "ws" ? 1 : kMlaDefaultVariant;
-  // the pair kernel reads q_nope 16 bytes at a time, the others 4: a view with an odd storage offset stays with those
-  if (variant == 2 && reinterpret_cast<uintptr_t>(q_nope.data_ptr()) % 16 != 0) variant = 1;
+  // A view into a larger buffer may start anywhere.  q_nope is read 16 bytes at a time by the pair kernel and 4 by the
+  // others, q_pe 4 by the lockstep kernel and 16 by the others; what the chosen kernel cannot read is copied first.  The cache
+  // comes in 16-byte pieces everywhere (the scales in the pair kernel in 4).
+  auto starts_at = [](const torch::Tensor& t, int bytes) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes == 0; };
+  if (!starts_at(q_nope, 4)) q_nope = q_nope.clone();
+  if (variant == 2 && !starts_at(q_nope, 16)) variant = 1;
+  if (!starts_at(q_pe, variant == 0 ? 4 : 16)) q_pe = q_pe.clone();
+  TORCH_CHECK(starts_at(ckv, 16) && starts_at(kpe, 16) && (variant == 2 || starts_at(scales, 16)),
+              "ckv / kpe (and scales, unless the pair kernel runs) must start on a 16-byte boundary");
   const int longest = (int)std::max<int64_t>(max_seq_len, 1);
   int nc = ctas > 0 ? (int)std::min<int64_t>(ctas, helix::kMlaMaxCtas)
            : variant == 2 ? helix::mla_pair_pick_ctas(B, longest, helix::device_sm_count())

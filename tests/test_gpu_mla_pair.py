@@ -94,3 +94,44 @@ def test_unaligned_queries_keep_a_kernel_that_takes_them(native_built):
     want, got = (attention.mla_decode(q, qp, ckv, scales, kpe, bt, sl, scale=0.07, max_seq_len=200) for q in (qn, shifted))
     # two kernels of the same precision: one bf16 rounding of values up to about 4.5 apart, and of the probabilities
     assert (want[0].float() - got[0].float()).abs().max() < 3e-2 and (want[1] - got[1]).abs().max() < 1e-3
+
+
+def _shift(t, elements):
+    """The same contiguous tensor, ``elements`` behind the start of its storage."""
+    flat = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)[elements:elements + t.numel()]
+    flat.copy_(t.reshape(-1))
+    return flat.view(t.shape)
+
+
+# q_nope and q_pe each 0, 2, 4 or 8 bytes off a 16-byte boundary: every kernel either reads them there or gets a copy
+@pytest.mark.parametrize("variant", ["pair", "ws", "lockstep"])
+@pytest.mark.parametrize("off_nope,off_pe", [(0, 1), (0, 2), (0, 4), (1, 0), (2, 2), (1, 1), (4, 4)])
+def test_queries_may_start_anywhere(native_built, monkeypatch, variant, off_nope, off_pe):
+    from helix_a2a_b200.ops import attention
+    monkeypatch.setenv("HELIX_A2A_MLA_VARIANT", variant)
+    qn, qp, ckv, scales, kpe, bt, sl = _case([200, 33], 16, seed=9)
+    want = attention.mla_decode(qn, qp, ckv, scales, kpe, bt, sl, scale=0.07, max_seq_len=200)
+    a, b = _shift(qn, off_nope), _shift(qp, off_pe)
+    assert a.data_ptr() % 16 == 2 * off_nope and b.data_ptr() % 16 == 2 * off_pe
+    got = attention.mla_decode(a, b, ckv, scales, kpe, bt, sl, scale=0.07, max_seq_len=200)
+    # as in the test above where another kernel of the same precision may have run, to the bit elsewhere
+    if variant == "pair" and off_nope in (2, 4):
+        assert (want[0].float() - got[0].float()).abs().max() < 3e-2 and (want[1] - got[1]).abs().max() < 1e-3
+    else:
+        assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+def test_a_cache_off_its_boundary_is_refused(native_built, monkeypatch):
+    from helix_a2a_b200.ops import attention
+    qn, qp, ckv, scales, kpe, bt, sl = _case([200, 33], 16, seed=9)
+    call = lambda c, s, k: attention.mla_decode(qn, qp, c, s, k, bt, sl, scale=0.07, max_seq_len=200)   # noqa: E731
+    want = call(ckv, scales, kpe)
+    with pytest.raises(RuntimeError, match="16-byte boundary"):
+        call(_shift(ckv.view(torch.uint8), 8).view(ckv.dtype), scales, kpe)
+    with pytest.raises(RuntimeError, match="16-byte boundary"):
+        call(ckv, scales, _shift(kpe, 2))
+    got = call(ckv, _shift(scales, 1), kpe)              # 4 bytes at a time in the pair kernel
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+    monkeypatch.setenv("HELIX_A2A_MLA_VARIANT", "ws")
+    with pytest.raises(RuntimeError, match="16-byte boundary"):
+        call(ckv, _shift(scales, 1), kpe)
