@@ -1,5 +1,6 @@
 // Torch bindings of the compute kernels (decode attention, o_proj GEMM).
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -32,19 +33,40 @@ bool env_pdl() {
 // stream: calls that may overlap on one GPU must be ordered by the caller).  Grown on demand, never shrunk; a
 // buffer that is outgrown is kept alive until the process ends, because a CUDA graph captured earlier may still
 // hold its address.  All kernels that use the counters leave them at zero.
+//
+// A call may be two launches (a streaming kernel and the fold of its partials) that meet in the scratch, so nothing of
+// another call may come between them on a stream that several threads share:
+//   * a call holds the device's scratch from taking it to its last launch (ScratchUse);
+//   * calls that are being captured have counters and partials of their own, because a graph that one thread replays
+//     may land between the two launches of another thread's eager call.  A graph itself is one unit of its stream.
 struct Scratch {
+  struct Set {
+    torch::Tensor counters;        // int32 [N]
+    torch::Tensor part_a, part_b;  // float32 pools
+  };
+  std::mutex launching;
   torch::Tensor error_flag;    // int32 [1]
-  torch::Tensor counters;      // int32 [N]
-  torch::Tensor part_a, part_b;  // float32 pools
-  torch::Tensor trace;           // int64 [rows * 8], only with one of the *_TRACE / *_PROF variables set
+  Set sets[2];                 // eager calls, captured calls
+  torch::Tensor trace;         // int64 [rows * 8], only with one of the *_TRACE / *_PROF variables set
   std::vector<torch::Tensor> retired;
 };
 std::mutex g_mu;
 std::map<int, Scratch> g_scratch;
 
-Scratch& scratch_for(const torch::Device& dev, int64_t counters, int64_t part_a_floats, int64_t part_b_floats) {
-  std::lock_guard<std::mutex> lk(g_mu);
-  Scratch& s = g_scratch[dev.index()];
+struct ScratchUse {
+  Scratch& dev;
+  Scratch::Set& set;
+  std::unique_lock<std::mutex> held;
+};
+
+ScratchUse scratch_for(const torch::Device& dev, int64_t counters, int64_t part_a_floats, int64_t part_b_floats) {
+  Scratch* entry;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    entry = &g_scratch[dev.index()];
+  }
+  Scratch& s = *entry;
+  std::unique_lock<std::mutex> held(s.launching);
   auto iopt = torch::TensorOptions().dtype(torch::kInt32).device(dev);
   auto fopt = torch::TensorOptions().dtype(torch::kFloat32).device(dev);
   auto grow = [&](torch::Tensor& t, int64_t need, int64_t floor, const torch::TensorOptions& opt, bool zero) {
@@ -54,10 +76,15 @@ Scratch& scratch_for(const torch::Device& dev, int64_t counters, int64_t part_a_
     t = zero ? torch::zeros({n}, opt) : torch::empty({n}, opt);
   };
   if (!s.error_flag.defined()) s.error_flag = torch::zeros({1}, iopt);
-  grow(s.counters, counters, 16384, iopt, true);
-  grow(s.part_a, part_a_floats, 1, fopt, false);
-  grow(s.part_b, part_b_floats, 1, fopt, false);
-  return s;
+  const bool captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  // An eager call grows both sets: what is captured after a warm-up finds its own ready, its counters zeroed by a memset
+  // that has run and is not part of the graph.
+  for (int i = captured ? 1 : 0; i < 2; ++i) {
+    grow(s.sets[i].counters, counters, 16384, iopt, true);
+    grow(s.sets[i].part_a, part_a_floats, 1, fopt, false);
+    grow(s.sets[i].part_b, part_b_floats, 1, fopt, false);
+  }
+  return {s, s.sets[captured ? 1 : 0], std::move(held)};
 }
 
 // Eight int64 stamps for each of `rows` CTAs.  A tensor that has become too small is kept like the other buffers.
@@ -158,7 +185,7 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   if (B == 0) return std::make_tuple(o, lse);
   const int max_helper = helix::kGqaMaxHelper;
   // the o_proj counters sit in the last hidden / 128 ints of the same tensor: leave them room
-  Scratch& sc = scratch_for(q.device(), (int64_t)helix::gqa_counter_ints(B * Hkv, max_helper) + 2048,
+  ScratchUse sc = scratch_for(q.device(), (int64_t)helix::gqa_counter_ints(B * Hkv, max_helper) + 2048,
                             (int64_t)helix::gqa_part_o_floats(sp, max_helper),
                             (int64_t)helix::gqa_part_lse_floats(sp, max_helper));
   helix::GqaDecodeParams p{};
@@ -172,10 +199,10 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   p.seq_lens = seq_lens.data_ptr<int32_t>();
   p.o = reinterpret_cast<__nv_bfloat16*>(o.data_ptr());
   p.lse = lse.data_ptr<float>();
-  p.part_o = sc.part_a.data_ptr<float>();
-  p.part_lse = sc.part_b.data_ptr<float>();
-  p.counters = sc.counters.data_ptr<int32_t>();
-  p.error_flag = sc.error_flag.data_ptr<int32_t>();
+  p.part_o = sc.set.part_a.data_ptr<float>();
+  p.part_lse = sc.set.part_b.data_ptr<float>();
+  p.counters = sc.set.counters.data_ptr<int32_t>();
+  p.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.page_size = page; p.ctas = sp;
   p.whole = splits <= 0 && helix::gqa_whole_pairs(B, Hkv, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
   // HELIX_A2A_ATTN_DYN_PCT / HELIX_A2A_ATTN_DYN_CHUNK: share of every long pair that is handed out dynamically
@@ -191,7 +218,7 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
     const char* tr = std::getenv("HELIX_A2A_ATTN_TRACE");
     if (tr && tr[0] == '1') {
       p.trace_rows = helix::gqa_grid(p);
-      p.trace = trace_for(sc, q.device(), p.trace_rows);
+      p.trace = trace_for(sc.dev, q.device(), p.trace_rows);
     }
   }
   p.kv_stable = kv_stable ? 1 : 0;
@@ -251,7 +278,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
            : variant == 2 ? helix::mla_pair_pick_ctas(B, longest, helix::device_sm_count())
                           : helix::mla_pick_ctas(B, longest, helix::device_sm_count());
   if (variant == 2) nc = std::max(nc / 2 * 2, 2);
-  Scratch& sc = scratch_for(q_nope.device(), (int64_t)B + 1024, (int64_t)helix::mla_part_o_floats(nc),
+  ScratchUse sc = scratch_for(q_nope.device(), (int64_t)B + 1024, (int64_t)helix::mla_part_o_floats(nc),
                             (int64_t)helix::mla_part_lse_floats(nc));
   helix::MlaDecodeParams p{};
   p.q_nope = reinterpret_cast<const __nv_bfloat16*>(q_nope.data_ptr());
@@ -264,10 +291,10 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   p.seq_lens = seq_lens.data_ptr<int32_t>();
   p.o = reinterpret_cast<__nv_bfloat16*>(o.data_ptr());
   p.lse = lse.data_ptr<float>();
-  p.part_o = sc.part_a.data_ptr<float>();
-  p.part_lse = sc.part_b.data_ptr<float>();
-  p.counters = sc.counters.data_ptr<int32_t>();
-  p.error_flag = sc.error_flag.data_ptr<int32_t>();
+  p.part_o = sc.set.part_a.data_ptr<float>();
+  p.part_lse = sc.set.part_b.data_ptr<float>();
+  p.counters = sc.set.counters.data_ptr<int32_t>();
+  p.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
   p.B = B; p.page_size = page; p.ctas = nc;
   p.scale = (float)scale;
   p.lse_base2 = lse_base2 ? 1 : 0;
@@ -276,7 +303,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
   p.prof = nullptr;
   {
     static const bool prof_on = [] { const char* v = std::getenv("HELIX_A2A_MLA_PROF"); return v && std::string(v) == "1"; }();
-    if (prof_on) p.prof = trace_for(sc, q_nope.device(), nc);
+    if (prof_on) p.prof = trace_for(sc.dev, q_nope.device(), nc);
   }
   check_cuda(helix::launch_mla_decode(p, env_pdl(), stream), "mla decode launch");
   return std::make_tuple(o, lse);
@@ -316,16 +343,16 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, sms);
     const int64_t part_floats = streamk ? (int64_t)helix::oproj_streamk_partial_floats(sk_ctas, n_pad)
                                         : (sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0);
-    Scratch& sc = scratch_for(x.device(), hidden / 128 + 1024, part_floats, 0);
+    ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024, part_floats, 0);
     helix::OprojParams p{};
     p.w_map = mat_map(w, 128);
     p.x_map = mat_map(xs, n_pad);
     p.y = reinterpret_cast<__nv_bfloat16*>(y.data_ptr()) + (int64_t)t0 * y.stride(0);
     p.y_stride = y.stride(0);
-    p.partial = sc.part_a.data_ptr<float>();
+    p.partial = sc.set.part_a.data_ptr<float>();
     // o_proj counters live after the attention counters
-    p.counters = sc.counters.data_ptr<int32_t>() + (sc.counters.numel() - hidden / 128);
-    p.error_flag = sc.error_flag.data_ptr<int32_t>();
+    p.counters = sc.set.counters.data_ptr<int32_t>() + (sc.set.counters.numel() - hidden / 128);
+    p.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
     p.tokens = nt; p.n_pad = n_pad; p.hidden = hidden; p.K = K; p.splits = sp;
     p.stages = helix::oproj_pick_stages(n_pad);
     p.atoms = helix::oproj_pick_atoms(n_pad);
@@ -334,7 +361,7 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     p.trace = nullptr;
     if (streamk) {
       static const bool trace_on = [] { const char* v = std::getenv("HELIX_A2A_OPROJ_TRACE"); return v && std::string(v) == "1"; }();
-      if (trace_on) p.trace = trace_for(sc, x.device(), sk_ctas);
+      if (trace_on) p.trace = trace_for(sc.dev, x.device(), sk_ctas);
     }
     check_cuda(streamk          ? helix::launch_oproj_streamk(p, env_pdl(), stream)
                : plan.slabs > 0 ? helix::launch_oproj_split(p, plan.slabs, env_pdl(), stream)
@@ -368,7 +395,7 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     const helix::OprojSplitPlan plan = sp <= 0 ? helix::oproj_pick_split_plan(hidden, K, n_pad, helix::device_sm_count())
                                                : helix::OprojSplitPlan{0, 0};
     if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, helix::device_sm_count());
-    Scratch& sc = scratch_for(x.device(), hidden / 128 + 1024,
+    ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024,
                               sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0, 0);
     helix::OprojParams p{};
     p.x_map = mat_map(xs, n_pad);
@@ -377,9 +404,9 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     p.packed_atoms = helix::oproj_packed_atoms(K);
     p.y = reinterpret_cast<__nv_bfloat16*>(y.data_ptr()) + (int64_t)t0 * y.stride(0);
     p.y_stride = y.stride(0);
-    p.partial = sc.part_a.data_ptr<float>();
-    p.counters = sc.counters.data_ptr<int32_t>() + (sc.counters.numel() - hidden / 128);
-    p.error_flag = sc.error_flag.data_ptr<int32_t>();
+    p.partial = sc.set.part_a.data_ptr<float>();
+    p.counters = sc.set.counters.data_ptr<int32_t>() + (sc.set.counters.numel() - hidden / 128);
+    p.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
     p.tokens = nt; p.n_pad = n_pad; p.hidden = hidden; p.K = K; p.splits = sp;
     p.stages = helix::oproj_pick_stages(n_pad);
     p.atoms = helix::oproj_pick_atoms(n_pad);
@@ -391,9 +418,9 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
 }
 
 torch::Tensor attn_trace(torch::Tensor like) {
-  Scratch& sc = scratch_for(like.device(), 1, 0, 0);
-  TORCH_CHECK(sc.trace.defined(), "no trace recorded: set HELIX_A2A_ATTN_TRACE=1 (or HELIX_A2A_OPROJ_TRACE=1)");
-  return sc.trace.clone();
+  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  TORCH_CHECK(sc.dev.trace.defined(), "no trace recorded: set HELIX_A2A_ATTN_TRACE=1 (or HELIX_A2A_OPROJ_TRACE=1)");
+  return sc.dev.trace.clone();
 }
 
 
@@ -448,14 +475,14 @@ std::tuple<torch::Tensor, torch::Tensor> fused_impl(torch::Tensor attn_out, torc
   torch::Tensor y = torch::empty(ys, attn_out.options());
   const int n_pad = (int)((B + 15) / 16 * 16);
   const int64_t part_floats = splits > 1 ? (int64_t)helix::oproj_partial_bytes((int)hidden, splits, n_pad) / 4 * ranks : 0;
-  Scratch& sc = scratch_for(attn_out.device(), (hidden / 128 + helix::fused_aux_ints((int)hidden)) * ranks + 1024, part_floats, 0);
+  ScratchUse sc = scratch_for(attn_out.device(), (hidden / 128 + helix::fused_aux_ints((int)hidden)) * ranks + 1024, part_floats, 0);
 
   helix::FusedParams fp{};
   helix::ExchangeParams& p = fp.ex;
   {
     // per-CTA %globaltimer stamps of the one-kernel path (read back with attn_trace)
     static const bool trace_on = [] { const char* v = std::getenv("HELIX_A2A_EXCHANGE_TRACE"); return v && std::string(v) == "1"; }();
-    if (trace_on) p.trace = trace_for(sc, attn_out.device(), helix::kGqaMaxCtas);
+    if (trace_on) p.trace = trace_for(sc.dev, attn_out.device(), helix::kGqaMaxCtas);
   }
   for (int r = 0; r < ranks; ++r) {
     p.io[r].o_src = reinterpret_cast<const uint8_t*>(attn_out.data_ptr()) + (int64_t)r * B * H * D * 2;
@@ -475,14 +502,14 @@ std::tuple<torch::Tensor, torch::Tensor> fused_impl(torch::Tensor attn_out, torc
     g.y = reinterpret_cast<__nv_bfloat16*>(y.data_ptr()) + (int64_t)r * B * hidden;
     g.y_stride = hidden;
     // every emulated rank needs its own split partials and slab counters
-    g.partial = splits > 1 ? sc.part_a.data_ptr<float>() + (int64_t)r * (part_floats / ranks) : nullptr;
+    g.partial = splits > 1 ? sc.set.part_a.data_ptr<float>() + (int64_t)r * (part_floats / ranks) : nullptr;
     {
       // from the end of the counter buffer: [slab counters | aux] per rank, all zero between calls
       const int64_t per_rank = hidden / 128 + helix::fused_aux_ints((int)hidden);
-      g.counters = sc.counters.data_ptr<int32_t>() + (sc.counters.numel() - per_rank * (r + 1));
+      g.counters = sc.set.counters.data_ptr<int32_t>() + (sc.set.counters.numel() - per_rank * (r + 1));
       fp.aux[r] = g.counters + hidden / 128;
     }
-    g.error_flag = sc.error_flag.data_ptr<int32_t>();
+    g.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
     g.tokens = (int)B; g.n_pad = n_pad; g.hidden = (int)hidden; g.K = (int)K; g.splits = splits;
     g.timeout_ns = timeout_ms > 0 ? (unsigned long long)timeout_ms * 1000000ull : env_timeout_ns();
   }
@@ -531,14 +558,14 @@ bool fused_oproj_fits(int64_t tokens, int64_t heads_local, int64_t head_dim, int
 }
 
 int64_t read_error_flag(torch::Tensor like) {
-  Scratch& sc = scratch_for(like.device(), 1, 0, 0);
-  return sc.error_flag.item<int>();
+  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  return sc.dev.error_flag.item<int>();
 }
 
 void clear_error_flag(torch::Tensor like) {
-  Scratch& sc = scratch_for(like.device(), 1, 0, 0);
-  sc.error_flag.zero_();
-  sc.counters.zero_();
+  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  sc.dev.error_flag.zero_();
+  for (Scratch::Set& set : sc.dev.sets) set.counters.zero_();
 }
 
 }  // namespace

@@ -12,11 +12,12 @@
 // supply is the kernel's private scratch (per-CTA partial results and arrival counters of the
 // split-KV merge), so here that scratch lives inside the library image.
 //
-// The scratch is ONE file-scope device array of fixed size (about 5.3 MB, see the limits below).
-// Every GPU that loads the library carries it from load until the process ends.  All calls on a
-// device share it, and it keeps whatever the previous call left behind: the entry point clears the
-// parts that must start at zero (arrival counters, error word) on the caller's stream before each
-// launch.  Because the array is shared, two calls whose kernels may overlap on the same GPU (for
+// The scratch is ONE file-scope device array of fixed size (about 10.6 MB, see the limits below).
+// Every GPU that loads the library carries it from load until the process ends.  All eager calls on
+// a device share one half of it and all calls captured into CUDA graphs the other, and it keeps
+// whatever the previous call left behind: the entry point clears the parts that must start at zero
+// (arrival counters, error word) on the caller's stream before each launch.  Threads may call on one
+// stream.  Because the array is shared, two calls whose kernels may overlap on the same GPU (for
 // instance on different streams) race on it; callers must order such calls themselves.
 //
 // The first call on each device performs a one-time set-up (it resolves the device address of the

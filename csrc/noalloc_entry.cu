@@ -16,16 +16,21 @@
 
 namespace {
 
-// Layout of the built-in scratch (bytes):
+// Layout of the built-in scratch (bytes): two sets, one for eager and one for captured calls, then the error word.
+// A set:
 //   [0, kPartO)                    partial outputs   [MAX_CTAS][2][8][128] fp32
 //   [kPartO, kPartO + kPartL)      partial LSEs      [MAX_CTAS][2][8]      fp32
 //   then                           arrival counters  [MAX_PAIRS]           int32   (must be zero at launch)
-//   then                           error word        int32 (+ padding)             (must be zero at launch)
+// Error word: int32 (+ padding), must be zero at launch.
+// A call is up to two launches that meet in its set, so it holds the device's lock from the first to the last (threads
+// may share a stream), and a graph that one thread replays between the launches of another's eager call finds its own set.
 constexpr size_t kPartO = (size_t)HELIX_NOALLOC_MAX_CTAS * 2 * 8 * 128 * sizeof(float);
 constexpr size_t kPartL = (size_t)HELIX_NOALLOC_MAX_CTAS * 2 * 8 * sizeof(float);
 constexpr size_t kCounters = (size_t)HELIX_NOALLOC_MAX_PAIRS * sizeof(int);
 constexpr size_t kErr = 256;
-constexpr size_t kScratchBytes = kPartO + kPartL + kCounters + kErr;
+constexpr size_t kSetBytes = kPartO + kPartL + kCounters, kErrAt = 2 * kSetBytes;
+constexpr size_t kScratchBytes = kErrAt + kErr;
+static_assert(kSetBytes % 256 == 0, "both sets are aligned alike");
 static_assert(HELIX_NOALLOC_MAX_CTAS <= helix::kGqaMaxCtas, "the kernel's grid bound sizes the piece slots");
 static_assert(kPartO == helix::gqa_part_o_floats(HELIX_NOALLOC_MAX_CTAS, 0) * sizeof(float) &&
                   kPartL == helix::gqa_part_lse_floats(HELIX_NOALLOC_MAX_CTAS, 0) * sizeof(float),
@@ -39,6 +44,7 @@ struct DeviceState {
   bool ready = false;
   unsigned char* base = nullptr;
   int sm_count = 0;
+  std::mutex launching;
 };
 DeviceState g_state[64];
 std::mutex g_mu;
@@ -122,7 +128,10 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
     return kHelixNoAllocBadArgument;
   int ctas = helix::gqa_pick_ctas(batch, kv_heads, max_seq_len > 0 ? max_seq_len : 1, st->sm_count);
   if (ctas > HELIX_NOALLOC_MAX_CTAS) ctas = HELIX_NOALLOC_MAX_CTAS;
-  unsigned char* base = st->base;
+  std::lock_guard<std::mutex> launching(st->launching);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) (void)cudaGetLastError();     // the launch below reports it
+  unsigned char* base = st->base + (capture == cudaStreamCaptureStatusNone ? 0 : kSetBytes);
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.q_stride_b = q_stride_batch;
   p.q_stride_h = q_stride_head;
@@ -134,7 +143,7 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
   p.part_o = reinterpret_cast<float*>(base);
   p.part_lse = reinterpret_cast<float*>(base + kPartO);
   p.counters = reinterpret_cast<int*>(base + kPartO + kPartL);
-  p.error_flag = reinterpret_cast<int*>(base + kPartO + kPartL + kCounters);
+  p.error_flag = reinterpret_cast<int*>(st->base + kErrAt);
   p.trace = nullptr;
   p.B = batch;
   p.Hq = q_heads;
@@ -165,7 +174,7 @@ extern "C" __attribute__((visibility("default"))) int helix_noalloc_read_error(v
   if (setup_current_device(&st) != kHelixNoAllocOk) return -1;
   int v = 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemcpyAsync(&v, st->base + kPartO + kPartL + kCounters, sizeof(int), cudaMemcpyDeviceToHost, s) !=
+  if (cudaMemcpyAsync(&v, st->base + kErrAt, sizeof(int), cudaMemcpyDeviceToHost, s) !=
           cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return -1;
