@@ -310,6 +310,25 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
 }
 
 // ---- o_proj ----------------------------------------------------------------------------------------
+// How one launch's worth of tokens (padded to n_pad) is run.  splits: 0 = pick (stream-K when it pays), -1 = force
+// stream-K, >= 1 = that many K splits of the plain kernel.  Packed weights have no stream-K form.
+struct OprojForm {
+  bool streamk;
+  helix::OprojSplitPlan plan;
+  int splits;
+  int launches() const { return plan.slabs > 0 && splits > 1 ? 2 : 1; }
+};
+OprojForm oproj_form(int hidden, int K, int n_pad, int64_t splits, bool packed, int sms) {
+  OprojForm f{!packed && (splits == -1 || (splits == 0 && helix::oproj_streamk_pays(hidden, K, n_pad, sms))), {0, 0}, (int)splits};
+  if (splits == 0 && !packed) {
+    // HELIX_A2A_OPROJ_STREAMK=1 / 0 overrides the choice for calls that leave it to the library
+    if (const char* v = std::getenv("HELIX_A2A_OPROJ_STREAMK")) f.streamk = std::string(v) == "1";
+  }
+  if (!f.streamk && (splits == 0 || (packed && splits < 0))) f.plan = helix::oproj_pick_split_plan(hidden, K, n_pad, sms);
+  if (splits <= 0) f.splits = f.plan.slabs > 0 ? f.plan.splits : helix::oproj_pick_splits(hidden, K, sms);
+  return f;
+}
+
 torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda(), "inputs must be on CUDA");
   TORCH_CHECK(x.scalar_type() == at::ScalarType::BFloat16 && w.scalar_type() == at::ScalarType::BFloat16,
@@ -328,19 +347,13 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     const int nt = std::min(256, tokens - t0);
     torch::Tensor xs = x.narrow(0, t0, nt);
     const int n_pad = (nt + 15) / 16 * 16;
-    int sp = (int)splits;
     const int sms = helix::device_sm_count();
-    // splits: 0 = pick (stream-K when it pays), -1 = force stream-K, >= 1 = that many K splits
-    bool streamk = sp == -1 || (sp == 0 && helix::oproj_streamk_pays(hidden, K, n_pad, sms));
-    if (sp == 0) {
-      // HELIX_A2A_OPROJ_STREAMK=1 / 0 overrides the choice for calls that leave it to the library
-      if (const char* v = std::getenv("HELIX_A2A_OPROJ_STREAMK")) streamk = std::string(v) == "1";
-    }
+    const OprojForm form = oproj_form(hidden, K, n_pad, splits, false, sms);
+    const helix::OprojSplitPlan plan = form.plan;
+    const bool streamk = form.streamk;
+    const int sp = form.splits;
     const int bk = 64 * helix::oproj_pick_atoms(n_pad);
     const int sk_ctas = (int)std::min<int64_t>(sms, (int64_t)(hidden / 128) * ((K + bk - 1) / bk));
-    const helix::OprojSplitPlan plan = sp == 0 && !streamk ? helix::oproj_pick_split_plan(hidden, K, n_pad, sms)
-                                                           : helix::OprojSplitPlan{0, 0};
-    if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, sms);
     const int64_t part_floats = streamk ? (int64_t)helix::oproj_streamk_partial_floats(sk_ctas, n_pad)
                                         : (sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0);
     ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024, part_floats, 0);
@@ -391,10 +404,9 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     const int nt = std::min(256, tokens - t0);
     torch::Tensor xs = x.narrow(0, t0, nt);
     const int n_pad = (nt + 15) / 16 * 16;
-    int sp = (int)splits;
-    const helix::OprojSplitPlan plan = sp <= 0 ? helix::oproj_pick_split_plan(hidden, K, n_pad, helix::device_sm_count())
-                                               : helix::OprojSplitPlan{0, 0};
-    if (sp <= 0) sp = plan.slabs > 0 ? plan.splits : helix::oproj_pick_splits(hidden, K, helix::device_sm_count());
+    const OprojForm form = oproj_form(hidden, K, n_pad, splits, true, helix::device_sm_count());
+    const helix::OprojSplitPlan plan = form.plan;
+    const int sp = form.splits;
     ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024,
                               sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0, 0);
     helix::OprojParams p{};
@@ -557,6 +569,17 @@ bool fused_oproj_fits(int64_t tokens, int64_t heads_local, int64_t head_dim, int
   return helix::fused_fits((int)tokens, (int)heads_local, (int)head_dim, (int)hidden, (int)cp_size, helix::device_sm_count());
 }
 
+// Kernels one call of the op launches when the form is left to the library.
+int gqa_launches(int B, int Hkv, int max_seq_len, int sm_count) {
+  return B <= 0 ? 0 : helix::gqa_whole_pairs(B, Hkv, std::max(max_seq_len, 1), sm_count) ? 1 : 2;
+}
+int oproj_launches(int tokens, int hidden, int K, bool packed, int sm_count) {
+  int n = 0;
+  for (int t0 = 0; t0 < tokens; t0 += 256)
+    n += oproj_form(hidden, K, (std::min(256, tokens - t0) + 15) / 16 * 16, 0, packed, sm_count).launches();
+  return n;
+}
+
 int64_t read_error_flag(torch::Tensor like) {
   ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
   return sc.dev.error_flag.item<int>();
@@ -597,5 +620,7 @@ void register_compute_ops(torch::Library& m) {
 void bind_compute(pybind11::module_& m) {
   m.def("gqa_pick_ctas", &helix::gqa_pick_ctas);
   m.def("oproj_pick_splits", &helix::oproj_pick_splits);
+  m.def("gqa_launches", &gqa_launches);
+  m.def("oproj_launches", &oproj_launches);
   m.def("fused_oproj_fits", &fused_oproj_fits);
 }

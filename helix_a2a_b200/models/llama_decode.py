@@ -22,6 +22,7 @@ import torch.distributed as dist
 
 from .. import api
 from ..ops import attention, oproj as oproj_mod
+from ..ops._ext import ext
 from ..utils import env
 from ..utils.tracing import nvtx_range
 
@@ -212,7 +213,16 @@ class HelixDecodeStack:
 
     # ---- accounting ------------------------------------------------------------------------------
     def kernels_per_step(self) -> int:
-        return self.cfg.n_layers * ((2 if self.fuse_oproj else 3) if self.cp_size > 1 else 2)
+        """Kernels of this library that one step launches (a split attention or o_proj call is two); counted for a GPU of 148
+        SMs where the stack is not on one."""
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 148
+        attn = ext().gqa_launches(self.batch, self.cfg.n_kv_heads, self.local_ctx, sms)
+        if self.cp_size > 1 and self.fuse_oproj:
+            return self.cfg.n_layers * (attn + 1)
+        packed = self.prepack_oproj and self.cfg.hidden % 128 == 0 and self.k_local % 64 == 0
+        own = packed or not oproj_mod.library_gemm_pays(self.batch, self.k_local)
+        proj = ext().oproj_launches(self.batch, self.cfg.hidden, self.k_local, packed, sms) if own else 0
+        return self.cfg.n_layers * (attn + (1 if self.cp_size > 1 else 0) + proj)
 
     def h2d_bytes_per_step(self) -> int:
         c = self.cfg

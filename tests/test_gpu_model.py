@@ -67,3 +67,22 @@ def test_mla_decode_stack_matches_oracle(native_built):
         outs.append(o)
     ref = rm.oproj_reference(torch.cat(outs).reshape(2, -1).bfloat16(), stack.w_o[l])
     assert (y.float() - ref).abs().max() < 5e-2 * max(1.0, ref.abs().max().item())
+
+
+# unsplit and split attention, o_proj as one launch, as two, and in slices of 256 tokens
+@pytest.mark.parametrize("batch,ctx,hidden", [(1, 300, 512), (1, 9000, 8192), (2, 20000, 512), (64, 100, 512), (300, 64, 2048)])
+def test_kernels_per_step_counts_what_is_launched(native_built, monkeypatch, batch, ctx, hidden):
+    from torch.profiler import ProfilerActivity, profile
+
+    from helix_a2a_b200.models.llama_decode import HelixDecodeStack, LlamaDecodeConfig
+    monkeypatch.delenv("HELIX_A2A_OPROJ_PREPACK", raising=False)
+    cfg = LlamaDecodeConfig.tiny(hidden=hidden, n_q_heads=64, n_kv_heads=8)
+    stack = HelixDecodeStack(cfg, batch=batch, local_ctx=ctx, device="cuda")
+    q = torch.randn(cfg.n_layers, batch, cfg.n_q_heads, cfg.head_dim, device="cuda").bfloat16()
+    stack.decode_step(q)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        stack.decode_step(q)
+        torch.cuda.synchronize()
+    ours = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA and "helix::" in e.name]
+    assert len(ours) == stack.kernels_per_step(), sorted(set(ours))
