@@ -24,7 +24,8 @@ struct GqaDecodeParams {
   __nv_bfloat16* o;            // [B, Hq, 128]
   float* lse;                  // [B, Hq]
   float* part_o;               // scratch [2 * ctas + max_helper][8][128] fp32: piece slots
-  float* part_lse;             // scratch [2 * ctas + max_helper][8]
+  float* part_lse;             // scratch [2 * ctas + max_helper][8], behind it int4 [ctas]: the split pair that a CTA's fixed
+                               // share starts, {pair or -1, CTA that ends its fixed part, chunks in its pool, their first slot}
   // scratch, zero on entry and zero again on exit (gqa_counter_ints(B * Hkv, max_helper) ints):
   //   [0, P)          blocks of the fold that have read the flags of a (sequence, kv head) pair
   //   [P, 2P)         chunks drawn from each pair's dynamic pool          (touched only when dyn_pct > 0)
@@ -56,7 +57,8 @@ constexpr int kGqaSeqTable = 256;    // batches beyond this run with fixed share
 
 // scratch sizes
 constexpr size_t gqa_part_o_floats(int ctas, int max_helper) { return ((size_t)ctas * 2 + max_helper) * 8 * 128; }
-constexpr size_t gqa_part_lse_floats(int ctas, int max_helper) { return ((size_t)ctas * 2 + max_helper) * 8; }
+constexpr size_t gqa_starts_at(int ctas, int max_helper) { return ((size_t)ctas * 2 + max_helper) * 8; }     // in part_lse
+constexpr size_t gqa_part_lse_floats(int ctas, int max_helper) { return gqa_starts_at(ctas, max_helper) + (size_t)ctas * 4; }
 constexpr size_t gqa_counter_ints(int pairs, int max_helper) { return (size_t)2 * pairs + 8 + max_helper; }
 
 // CTAs of the streaming launch: at most kGqaMaxCtas when pairs are split, but as many as there are pairs when they are whole

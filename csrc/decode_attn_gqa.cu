@@ -57,6 +57,8 @@ constexpr int kMaxList = 2048;                          // pieces one fold can l
 constexpr int kMaxPoolChunks = kMaxList - kGqaMaxCtas;   // chunks one pair's pool may hold: a fold lists at most one piece
                                                         // per CTA plus one per chunk of the pair
 static_assert(kMaxPoolChunks > 0, "the piece list must hold one piece per CTA");
+constexpr int kPlanPairs = 64;                          // up to so many pairs the fold works out by itself what to fold
+constexpr int kSerialSeqs = 16;                         // batches up to this size are planned by every thread on its own
 constexpr int kMinShare = 8, kWholeBlocks = 96, kWholeExtra = 40;      // 16-token blocks, see gqa_pick_ctas
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -83,6 +85,23 @@ __host__ __device__ __forceinline__ int dyn_chunks_of(int nb, int pct, int chunk
 __device__ __forceinline__ int ld_relaxed(const int* p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <class T>
+__device__ __forceinline__ T warp_sum(T v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// sum over this lane and all lanes below
+template <class T>
+__device__ __forceinline__ T warp_scan(T v) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T below = __shfl_up_sync(0xffffffffu, v, o);
+    if ((int)(threadIdx.x & 31) >= o) v += below;
+  }
   return v;
 }
 
@@ -151,6 +170,59 @@ __device__ __forceinline__ PairPlan plan_pair(const GqaDecodeParams& p, int b, i
   return pl;
 }
 
+// Planning of a launch with many sequences: every lane takes a run of them and shuffles join the runs (all warps alike,
+// warp 0 writes the tables).  When every thread walked all sequences, three times, that was a quarter of the streaming kernel
+// for 128 sequences of 16 tokens (8 kv heads, a bound that keeps them in shares): 44.9 -> 34.1 us; 512 tokens 74.5 -> 63.0.
+// Up to kSerialSeqs sequences the walk is as fast.  Out of line: inside the kernel it costs the launches that do not need it
+// 0.2 us of instruction fetch.
+struct ManyPlan {
+  long long total;       // blocks in the fixed shares
+  long long base;        // share-space index of the first block of sequence b, at or a few sequences before this CTA's share
+  int b;
+  bool pools;            // some pair has a pool
+};
+__device__ __noinline__ ManyPlan plan_many(const GqaDecodeParams& p, const int* s_nb, const unsigned short* s_nc,
+                                           unsigned short* s_ncf, int* s_hb) {
+  const int lane = threadIdx.x & 31, G = gridDim.x, Hkv = p.Hkv, n_tab = min(p.B, kGqaSeqTable);
+  const int run = (n_tab + 31) / 32, lo = min(lane * run, n_tab), hi = min(lo + run, n_tab);
+  long long rest = 0, total = 0;                 // sequences behind the table; all of them
+  for (int b = kGqaSeqTable + lane; b < p.B; b += 32) rest += blocks_of(p.seq_lens[b]);
+  for (int b = lo; b < hi; ++b) total += s_nb[b];
+  rest = warp_sum(rest);
+  total = warp_sum(total) + rest;
+  const long long share_max = (total * Hkv + G - 1) / G + 1;
+  int want = 0;
+  for (int b = lo; b < hi; ++b) want += pool_chunks(p, s_nb[b], s_nc[b], share_max, 0);
+  int hb = warp_scan(want) * Hkv;
+  if (__shfl_sync(0xffffffffu, hb, 31) <= p.max_helper) {
+    hb -= want * Hkv;
+  } else {                                       // not every pair gets its chunks: who does depends on those before
+    hb = 0;
+    for (int b = 0; b < lo; ++b) hb += pool_chunks(p, s_nb[b], s_nc[b], share_max, hb) * Hkv;
+  }
+  long long fixed = 0;
+  for (int b = lo; b < hi; ++b) {
+    const int nb = s_nb[b], nc = pool_chunks(p, nb, s_nc[b], share_max, hb);
+    if (threadIdx.x < 32) {
+      s_ncf[b] = (unsigned short)nc;
+      s_hb[b] = hb;
+    }
+    hb += nc * Hkv;
+    fixed += nb - nc * p.dyn_chunk;
+  }
+  const long long end = warp_scan(fixed), table = __shfl_sync(0xffffffffu, end, 31);
+  ManyPlan pl;
+  pl.total = (table + rest) * Hkv;
+  pl.pools = __shfl_sync(0xffffffffu, hb, 31) > 0;
+  // the run that holds the first block of this CTA's share, or the sequences behind the table
+  const long long g0 = (long long)blockIdx.x * max((pl.total + G - 1) / (long long)G, 1LL);
+  const unsigned holds = __ballot_sync(0xffffffffu, g0 < end * Hkv);
+  const int src = holds != 0 ? __ffs(holds) - 1 : 31;
+  pl.b = holds != 0 ? __shfl_sync(0xffffffffu, lo, src) : n_tab;
+  pl.base = (holds != 0 ? __shfl_sync(0xffffffffu, end - fixed, src) : table) * Hkv;
+  return pl;
+}
+
 // kTrace: the instance that records time stamps (the stamps cost registers the streaming loop needs)
 template <bool kTrace>
 __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_constant__ GqaDecodeParams p) {
@@ -200,10 +272,19 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   }
   __syncthreads();
   long long total_s = 0;                         // blocks in the fixed shares
-  if (!p.whole) {
+  int cur_b = 0;
+  long long base = 0;                            // share-space index of block 0 of (cur_b, kvh = 0)
+  if (p.whole) {
+    // CTA = pair
+  } else if (n_tab > kSerialSeqs) {
+    const ManyPlan pl = plan_many(p, s_nb, s_nc, s_ncf, s_hb);
+    total_s = pl.total;
+    cur_b = pl.b;
+    base = pl.base;
+    dyn_on = pl.pools;
+  } else {
     long long total = 0;
     for (int b = 0; b < n_tab; ++b) total += s_nb[b];
-    for (int b = kGqaSeqTable; b < p.B; ++b) total += blocks_of(p.seq_lens[b]);
     const long long share_max = (total * Hkv + G - 1) / G + 1;
     int hb = 0;
     for (int b = 0; b < n_tab; ++b) {
@@ -216,7 +297,6 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
       hb += nc * Hkv;
       total_s += nb - nc * cd;
     }
-    for (int b = kGqaSeqTable; b < p.B; ++b) total_s += blocks_of(p.seq_lens[b]);
     total_s *= Hkv;
     dyn_on = hb > 0;
   }
@@ -247,8 +327,6 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
     int slot;                // piece slot, should this segment open a new running state
     bool valid;
   };
-  int cur_b = 0;
-  long long base = 0;        // share-space index of block 0 of (cur_b, kvh = 0)
   while (!p.whole && cur_b < p.B) {
     const long long span = (long long)seq_ns(cur_b) * Hkv;
     if (g0 < base + span) break;
@@ -391,6 +469,9 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   } else if (cur.valid) {
     prologue(cur);
   }
+  int4* const start = reinterpret_cast<int4*>(p.part_lse + gqa_starts_at(G, p.max_helper)) + blockIdx.x;
+  const bool note_starts = !p.whole && P > kPlanPairs;
+  if (note_starts && tid == 0) start->x = -1;
   bool in_static = cur.valid;
   if (!cur.valid && dyn_on) {          // no fixed share (more CTAs than blocks): go straight to the pools
     cur = scan_pools(blockIdx.x % max(P, 1), false, false);
@@ -449,6 +530,10 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
     const int my_first = kb_begin + warp;
     const int my_count = my_first < kb_end ? (kb_end - my_first + kWarps - 1) / kWarps : 0;
     int next_page = kStages < my_count ? page_of(my_first + kStages * kWarps) : 0;
+    if (note_starts && in_static && tid == 0 && kb_begin == 0 && kb_end < seq_ns(b)) {
+      // the last pair of the share, continued by the next CTAs: the fold finds it here (the first tiles are on their way)
+      *start = make_int4(b * Hkv + kvh, (int)((gcur - kb_end + seq_ns(b) - 1) / share), my_nc, my_nc > 0 ? s_hb[b] + kvh * my_nc : 0);
+    }
 
     for (int it = 0; it < my_count; ++it) {
       const int ring = it_ring + it;
@@ -659,7 +744,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   }
 }
 
-// Merges the pieces of every pair that more than one CTA streamed, one launch behind the streaming kernel: it
+// Merges the pieces of every pair that more than one CTA streamed (up to kPlanPairs pairs), one launch behind the streaming kernel: it
 // is resident early (its tables are ready before the pieces are) and then has every SM to read them, where a fold by
 // the CTA that finished a pair last had one SM read all of its pieces, eight per round trip, behind an acquire-release
 // atomic that takes ~4 us while HBM is saturated.  Block (pair, y) merges query heads y, y + gridDim.y, ... of
@@ -772,6 +857,116 @@ __global__ void __launch_bounds__(kFoldThreads) gqa_fold_kernel(const __grid_con
   }
 }
 
+// The same for more than kPlanPairs pairs.  Most blocks only start when the streaming kernel is done then, and 256 to 2400
+// of the blocks above took 8 to 30 us to find out what little there is to fold.  Block (c, y) reads what CTA c noted about
+// the one split pair that its share starts: every split pair starts in exactly one CTA.  Up to eight pieces are one round
+// trip, so each warp takes a head of its own.  From the end of the streaming kernel to the end of the fold: 128 x 16 tokens
+// 22.5 -> 1.6 us, 128 x 2000 17.6 -> 3.9, 24 ragged up to 9000 5.2 -> 4.5.  Up to 64 pairs the kernel above is ahead by 0.5 to
+// 1.5 us: its plan is ready before the pieces are, and the note is one more round trip.
+constexpr int kFoldWarps = kFoldThreads / 32, kFoldBatch = 8;
+__global__ void __launch_bounds__(kFoldThreads) gqa_fold_starts_kernel(const __grid_constant__ GqaDecodeParams p) {
+  struct Sum {
+    float M, L;
+    float4 acc;
+  };
+  __shared__ unsigned short s_list[kMaxList];
+  __shared__ Sum s_sum[kFoldWarps][32];
+  __shared__ int s_n, s_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = p.Hq / p.Hkv;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int4 start = __ldcg(reinterpret_cast<const int4*>(p.part_lse + gqa_starts_at(p.ctas, p.max_helper)) + blockIdx.x);
+  if (start.x < 0) return;
+  const int pair = start.x, n_fixed = start.y - (int)blockIdx.x + 1, nc = start.z, hb = start.w;
+  for (int i = tid; i < n_fixed; i += kFoldThreads) s_list[i] = (unsigned short)((blockIdx.x + i) * 2 + (i == 0 ? 1 : 0));
+  if (tid == 0) s_n = n_fixed;
+  __syncthreads();
+  if (nc > 0) {
+    int* const helper_flag = p.counters + (size_t)2 * p.B * p.Hkv + 8 + hb;
+    for (int c = tid; c < nc; c += kFoldThreads)
+      if (__ldcg(helper_flag + c) != 0) s_list[atomicAdd(&s_n, 1)] = (unsigned short)(2 * p.ctas + hb + c);
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(p.counters + pair, 1) == (int)gridDim.y - 1;
+    __syncthreads();
+    if (s_last) {                               // every block of the pair has read the flags
+      for (int c = tid; c < nc; c += kFoldThreads) helper_flag[c] = 0;
+      if (tid == 0) {
+        p.counters[(size_t)p.B * p.Hkv + pair] = 0;
+        p.counters[pair] = 0;
+      }
+    }
+  }
+  const int n = s_n, b = pair / p.Hkv, kvh = pair % p.Hkv;
+  auto store = [&](const Sum& f, int hg) {
+    const float inv = f.L > 0.f ? 1.f / f.L : 0.f;
+    const int64_t row = (int64_t)b * p.Hq + kvh * group + hg;
+    *(reinterpret_cast<uint2*>(p.o + row * kD) + lane) =
+        make_uint2(pack_bf16(f.acc.x * inv, f.acc.y * inv), pack_bf16(f.acc.z * inv, f.acc.w * inv));
+    if (lane == 0) {
+      const float lse2 = f.L > 0.f ? f.M + log2f(f.L) : -INFINITY;
+      p.lse[row] = p.lse_base2 ? lse2 : lse2 * kLn2;
+    }
+  };
+  // the pieces i0, i0 + step, ... of one head, kFoldBatch rows and their LSEs per round trip, with a running maximum
+  auto rows = [&](int i0, int step, int hg) {
+    float M = -INFINITY, L = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (; i0 < n; i0 += kFoldBatch * step) {
+      float4 v[kFoldBatch];
+      float l[kFoldBatch];
+#pragma unroll
+      for (int j = 0; j < kFoldBatch; ++j) {
+        const int i = i0 + j * step;
+        l[j] = -INFINITY;
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n) {
+          const size_t row = (size_t)s_list[i] * 8 + hg;
+          l[j] = __ldcg(p.part_lse + row);
+          v[j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + row * kD) + lane);
+        }
+      }
+      float top = M;
+#pragma unroll
+      for (int j = 0; j < kFoldBatch; ++j) top = fmaxf(top, l[j]);
+      const float keep = M == -INFINITY ? 0.f : fast_exp2(M - top);
+      M = top;
+      L *= keep;
+      acc = make_float4(acc.x * keep, acc.y * keep, acc.z * keep, acc.w * keep);
+#pragma unroll
+      for (int j = 0; j < kFoldBatch; ++j) {
+        const float w = l[j] == -INFINITY ? 0.f : fast_exp2(l[j] - top);
+        L += w;
+        acc.x += w * v[j].x;
+        acc.y += w * v[j].y;
+        acc.z += w * v[j].z;
+        acc.w += w * v[j].w;
+      }
+    }
+    return Sum{M, L, acc};
+  };
+  if (n <= kFoldBatch) {
+    for (int hg = blockIdx.y * kFoldWarps + warp; hg < group; hg += gridDim.y * kFoldWarps) store(rows(0, 1, hg), hg);
+    return;
+  }
+  for (int hg = blockIdx.y; hg < group; hg += gridDim.y) {
+    s_sum[warp][lane] = rows(warp, kFoldWarps, hg);
+    __syncthreads();
+    if (warp == 0) {
+      Sum f = s_sum[0][lane];
+      for (int w = 1; w < kFoldWarps; ++w) {
+        const Sum s = s_sum[w][lane];
+        const float top = fmaxf(f.M, s.M);
+        const float x = f.M == -INFINITY ? 0.f : fast_exp2(f.M - top), y = s.M == -INFINITY ? 0.f : fast_exp2(s.M - top);
+        f.M = top;
+        f.L = f.L * x + s.L * y;
+        f.acc = make_float4(f.acc.x * x + s.acc.x * y, f.acc.y * x + s.acc.y * y, f.acc.z * x + s.acc.z * y, f.acc.w * x + s.acc.w * y);
+      }
+      store(f, hg);
+    }
+    __syncthreads();                            // s_sum is free again
+  }
+}
+
 }  // namespace
 
 // Number of CTAs for a launch: two per SM, but never so many that a CTA streams fewer than 8 blocks (two per warp).
@@ -842,12 +1037,12 @@ cudaError_t launch_gqa_decode(const GqaDecodeParams& p, bool pdl, cudaStream_t s
                                      : cudaLaunchKernelEx(&cfg, gqa_decode_kernel<false>, p);
   if (e != cudaSuccess || p.whole) return e;
   // The fold is always chained to this launch; it waits for the whole grid before it reads a piece.
-  const int pairs = p.B * p.Hkv;
-  cfg.gridDim = dim3(pairs, std::max(1, std::min(p.Hq / p.Hkv, 1184 / pairs)), 1);
+  const int pairs = p.B * p.Hkv, blocks = pairs <= kPlanPairs ? pairs : p.ctas;
+  cfg.gridDim = dim3(blocks, std::max(1, std::min(p.Hq / p.Hkv, 1184 / blocks)), 1);
   cfg.blockDim = dim3(kFoldThreads, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gqa_fold_kernel, p);
+  return cudaLaunchKernelEx(&cfg, pairs <= kPlanPairs ? gqa_fold_kernel : gqa_fold_starts_kernel, p);
 }
 
 }  // namespace helix

@@ -19,13 +19,13 @@ namespace {
 // Layout of the built-in scratch (bytes): two sets, one for eager and one for captured calls, then the error word.
 // A set:
 //   [0, kPartO)                    partial outputs   [MAX_CTAS][2][8][128] fp32
-//   [kPartO, kPartO + kPartL)      partial LSEs      [MAX_CTAS][2][8]      fp32
+//   [kPartO, kPartO + kPartL)      partial LSEs      [MAX_CTAS][2][8]      fp32, and what each CTA notes for the fold (16 bytes)
 //   then                           arrival counters  [MAX_PAIRS]           int32   (must be zero at launch)
 // Error word: int32 (+ padding), must be zero at launch.
 // A call is up to two launches that meet in its set, so it holds the device's lock from the first to the last (threads
 // may share a stream), and a graph that one thread replays between the launches of another's eager call finds its own set.
 constexpr size_t kPartO = (size_t)HELIX_NOALLOC_MAX_CTAS * 2 * 8 * 128 * sizeof(float);
-constexpr size_t kPartL = (size_t)HELIX_NOALLOC_MAX_CTAS * 2 * 8 * sizeof(float);
+constexpr size_t kPartL = (size_t)HELIX_NOALLOC_MAX_CTAS * (2 * 8 + 4) * sizeof(float);
 constexpr size_t kCounters = (size_t)HELIX_NOALLOC_MAX_PAIRS * sizeof(int);
 constexpr size_t kErr = 256;
 constexpr size_t kSetBytes = kPartO + kPartL + kCounters, kErrAt = 2 * kSetBytes;

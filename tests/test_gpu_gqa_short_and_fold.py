@@ -57,3 +57,32 @@ def test_time_stamps_have_a_row_for_every_cta(native_built, monkeypatch, lens, h
     stamps = ops().attn_trace(q).view(-1, 8)
     assert stamps.shape[0] >= ctas and (stamps[:ctas, 3] >= stamps[:ctas, 0]).all() and (stamps[:ctas, 0] > 0).all()
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+# Batches around the sizes where planning changes: lanes take runs of sequences above 16, pools end above 256, the fold finds
+# its pairs through the CTAs that start them above 64 pairs.  A bound below the real lengths makes the pools want more
+# chunks than there are slots; one far above them keeps short sequences in shares.
+@pytest.mark.parametrize("B,hkv,top,bound", [(16, 4, 3000, 3000), (17, 4, 3000, 3000), (33, 2, 6000, 6000), (20, 8, 5000, 1600),
+                                             (40, 8, 900, 131072), (200, 2, 1500, 131072), (256, 1, 2500, 2500),
+                                             (257, 1, 2500, 2500), (300, 2, 700, 131072), (70, 1, 9000, 2000)])
+def test_many_sequences_in_shares_and_pools(native_built, monkeypatch, B, hkv, top, bound):
+    from helix_a2a_b200.ops import attention, reference_math as rm
+    from helix_a2a_b200.ops.oproj import check_compute_status
+    lens = [(i * 7919 + 13) % top for i in range(B)]
+    lens[B // 2], lens[-1], lens[0] = top, 0, top
+    q, k, v, bt, sl = _case(lens, hkv, 4, 16, "HND", B)
+    o_ref, l_ref = rm.paged_decode_attention_reference(q, k, v, bt, sl, 1 / math.sqrt(128), False)
+    live = sl > 0
+    for pct, chunk, least in (("30", "4", "8"), ("0", "4", "8"), (None, None, None)):
+        for name, val in (("PCT", pct), ("CHUNK", chunk), ("MIN_BLOCKS", least)):
+            if val is None:
+                monkeypatch.delenv("HELIX_A2A_ATTN_DYN_" + name, raising=False)
+            else:
+                monkeypatch.setenv("HELIX_A2A_ATTN_DYN_" + name, val)
+        for _ in range(2):
+            o, lse = attention.gqa_decode(q, k, v, bt, sl, max_seq_len=bound)
+        torch.cuda.synchronize()
+        check_compute_status(q)
+        assert (o.float() - o_ref.float()).abs().max() < 2e-2, pct
+        assert (lse[live] - l_ref[live]).abs().max() < 1e-3, pct
+        assert torch.isneginf(lse[~live]).all()
