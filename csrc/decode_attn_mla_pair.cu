@@ -808,6 +808,111 @@ __global__ void __launch_bounds__(kFoldCols * kFoldMaxGroups)
   }
 }
 
+// The same for more sequences than clusters: at most one split sequence per cluster, and most sequences have nothing to
+// fold.  With a block per sequence and four heads the device went through 4096 (128 sequences) to 19200 blocks to find that
+// out, 5 to 30 us.  Block (c, y) looks for the sequence that cluster c's tiles start and do not end; warp = head, lane = 4 x 4
+// columns, four pieces per round trip with a running maximum.
+constexpr int kStartsWarps = 4, kStartsBatch = 4;
+__global__ void __launch_bounds__(kStartsWarps * 32)
+    mla_pair_fold_starts_kernel(const __grid_constant__ MlaDecodeParams p, int n_clusters) {
+  __shared__ int s_warp[kStartsWarps], s_b, s_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = blockIdx.x, h = blockIdx.y * kStartsWarps + warp;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // every thread takes a run of sequences: `end` = tiles up to the end of its run
+  const int run = (p.B + (int)blockDim.x - 1) / (int)blockDim.x, lo = min(tid * run, p.B), hi = min(lo + run, p.B);
+  int mine = 0;
+  for (int b = lo; b < hi; ++b) mine += max((p.seq_lens[b] + kTile - 1) / kTile, 0);
+  int end = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int below = __shfl_up_sync(0xffffffffu, end, d);
+    if (lane >= d) end += below;
+  }
+  if (lane == 31) s_warp[warp] = end;
+  if (tid == 0) s_b = -1;
+  __syncthreads();
+  int total = 0;
+#pragma unroll
+  for (int w = 0; w < kStartsWarps; ++w) {
+    if (w < warp) end += s_warp[w];
+    total += s_warp[w];
+  }
+  const int chunk = max((total + n_clusters - 1) / n_clusters, 1), next = (c + 1) * chunk;      // the next cluster's first tile
+  if (next < end && next > end - mine) {       // it lies inside this run, behind its first tile
+    int first = end - mine, b = lo;
+    for (;; ++b) {
+      const int n = max((p.seq_lens[b] + kTile - 1) / kTile, 0);
+      if (next < first + n) {
+        if (first < next && first >= c * chunk) s_b = b, s_last = (first + n - 1) / chunk;
+        break;
+      }
+      first += n;
+    }
+  }
+  __syncthreads();
+  for (int b = blockIdx.y * n_clusters + c; b < p.B; b += n_clusters * gridDim.y) {
+    if (p.seq_lens[b] > 0) continue;                 // an empty sequence: zeros
+    uint4* dst = reinterpret_cast<uint4*>(p.o + (int64_t)b * kH * kDn);
+    for (int i = tid; i < kH * kDn / 8; i += blockDim.x) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+    p.lse[(int64_t)b * kH + tid] = -INFINITY;
+  }
+  static_assert(kStartsWarps * 32 == kH, "a thread per LSE of an empty sequence");
+  if (s_b < 0) return;
+  const int n = s_last - c + 1;
+  float M = -INFINITY, L = 0.f;
+  float4 acc[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = 0; i0 < n; i0 += kStartsBatch) {
+    float4 v[kStartsBatch][4];
+    float l[kStartsBatch];
+#pragma unroll
+    for (int k = 0; k < kStartsBatch; ++k) {
+      l[k] = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[k][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i0 + k < n) {
+        // the first piece starts its sequence (slot 1); every later one begins where its cluster begins (slot 0)
+        const size_t row = ((size_t)(c + i0 + k) * 2 + (i0 + k == 0 ? 1 : 0)) * kH + h;
+        l[k] = __ldcg(p.part_lse + row);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[k][j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + row * kDn) + lane + 32 * j);
+      }
+    }
+    float top = M;
+#pragma unroll
+    for (int k = 0; k < kStartsBatch; ++k) top = fmaxf(top, l[k]);
+    const float keep = M == -INFINITY ? 0.f : fast_exp2(M - top);
+    M = top;
+    L *= keep;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = make_float4(acc[j].x * keep, acc[j].y * keep, acc[j].z * keep, acc[j].w * keep);
+#pragma unroll
+    for (int k = 0; k < kStartsBatch; ++k) {
+      const float w = l[k] == -INFINITY ? 0.f : fast_exp2(l[k] - top);
+      L += w;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[j].x += w * v[k][j].x;
+        acc[j].y += w * v[k][j].y;
+        acc[j].z += w * v[k][j].z;
+        acc[j].w += w * v[k][j].w;
+      }
+    }
+  }
+  const float inv = L > 0.f ? 1.f / L : 0.f;
+  const int64_t out = (int64_t)s_b * kH + h;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    reinterpret_cast<uint2*>(p.o + out * kDn)[lane + 32 * j] =
+        make_uint2(pack_bf16(acc[j].x * inv, acc[j].y * inv), pack_bf16(acc[j].z * inv, acc[j].w * inv));
+  if (lane == 0) {
+    const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
+    p.lse[out] = p.lse_base2 ? lse2 : lse2 * kLn2;
+  }
+}
+
 }  // namespace
 
 int mla_pair_pick_ctas(int B, int max_seq_len, int sm_count) {
@@ -833,14 +938,20 @@ cudaError_t launch_mla_decode_pair(const MlaDecodeParams& p, bool pdl, cudaStrea
   e = cudaLaunchKernelEx(&cfg, mla_pair_kernel, p);
   if (e != cudaSuccess) return e;
   // The fold is always chained to this launch: it waits for the whole grid before it reads anything.
+  cfg.dynamicSmemBytes = 0;
+  cfg.numAttrs = 1;
+  const int n_clusters = p.ctas / 2;
+  if (p.B > n_clusters) {
+    cfg.gridDim = dim3(n_clusters, kH / kStartsWarps, 1);
+    cfg.blockDim = dim3(kStartsWarps * 32, 1, 1);
+    return cudaLaunchKernelEx(&cfg, mla_pair_fold_starts_kernel, p, n_clusters);
+  }
   // A block's heads follow one another, 2-3 us each, so it takes several only where one each would be more blocks than
   // the device holds at once (16 of them per SM).
   const int heads = p.B <= 18 ? 1 : p.B <= 37 ? 2 : 4;
   cfg.gridDim = dim3(p.B, kH / heads, 1);
   cfg.blockDim = dim3(kFoldCols * (p.B <= 4 ? 4 : p.B <= 9 ? 2 : 1), 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, mla_pair_fold_kernel, p, p.ctas / 2, heads);
+  return cudaLaunchKernelEx(&cfg, mla_pair_fold_kernel, p, n_clusters, heads);
 }
 
 }  // namespace helix

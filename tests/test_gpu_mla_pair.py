@@ -57,7 +57,10 @@ def _check(seq_lens, page, ctas, scale, base2=False, std=0.5, poison=False):
 @pytest.mark.parametrize("seq_lens,page,ctas", [
     ([1], 16, 0), ([64], 16, 0), ([15, 16, 17, 63, 64, 65], 16, 2), ([127, 0, 128, 129], 32, 4), ([300, 1, 700], 48, 6),
     ([1024], 64, 2), ([1000], 64, 32), ([5, 0, 64] * 70, 16, 0), ([2049, 640, 4096], 32, 10), ([20000], 16, 0),
-    ([2000] * 6, 16, 0), ([300, 900] * 10, 32, 0), ([700] * 40, 16, 0)])
+    ([2000] * 6, 16, 0), ([300, 900] * 10, 32, 0), ([700] * 40, 16, 0),
+    # more sequences than clusters (the fold goes by what the clusters noted), more than the table in shared memory holds
+    ([200, 0, 16] * 50, 16, 0), ([64] * 75, 16, 0), ([9000] + [40] * 80, 16, 0), ([130, 0, 64, 1] * 150, 16, 0),
+    ([500, 70, 900], 16, 2), ([33, 700, 20, 0, 260], 16, 4)])
 def test_pair_kernel_matches_fp32_reference(native_built, seq_lens, page, ctas):
     _check(seq_lens, page, ctas, 1.0 / math.sqrt(192))
 
