@@ -310,7 +310,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
 }
 
 // ---- o_proj ----------------------------------------------------------------------------------------
-// How one launch's worth of tokens (padded to n_pad) is run.  splits: 0 = pick (stream-K when it pays), -1 = force
+// How one launch's worth of tokens (at most 256) is run.  splits: 0 = pick (stream-K when it pays), -1 = force
 // stream-K, >= 1 = that many K splits of the plain kernel.  Packed weights have no stream-K form.
 struct OprojForm {
   bool streamk;
@@ -318,13 +318,14 @@ struct OprojForm {
   int splits;
   int launches() const { return plan.slabs > 0 && splits > 1 ? 2 : 1; }
 };
-OprojForm oproj_form(int hidden, int K, int n_pad, int64_t splits, bool packed, int sms) {
+OprojForm oproj_form(int hidden, int K, int tokens, int64_t splits, bool packed, int sms) {
+  const int n_pad = (tokens + 15) / 16 * 16;
   OprojForm f{!packed && (splits == -1 || (splits == 0 && helix::oproj_streamk_pays(hidden, K, n_pad, sms))), {0, 0}, (int)splits};
   if (splits == 0 && !packed) {
     // HELIX_A2A_OPROJ_STREAMK=1 / 0 overrides the choice for calls that leave it to the library
     if (const char* v = std::getenv("HELIX_A2A_OPROJ_STREAMK")) f.streamk = std::string(v) == "1";
   }
-  if (!f.streamk && (splits == 0 || (packed && splits < 0))) f.plan = helix::oproj_pick_split_plan(hidden, K, n_pad, sms);
+  if (!f.streamk && (splits == 0 || (packed && splits < 0))) f.plan = helix::oproj_pick_split_plan(hidden, K, tokens, sms);
   if (splits <= 0) f.splits = f.plan.slabs > 0 ? f.plan.splits : helix::oproj_pick_splits(hidden, K, sms);
   return f;
 }
@@ -348,7 +349,7 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     torch::Tensor xs = x.narrow(0, t0, nt);
     const int n_pad = (nt + 15) / 16 * 16;
     const int sms = helix::device_sm_count();
-    const OprojForm form = oproj_form(hidden, K, n_pad, splits, false, sms);
+    const OprojForm form = oproj_form(hidden, K, nt, splits, false, sms);
     const helix::OprojSplitPlan plan = form.plan;
     const bool streamk = form.streamk;
     const int sp = form.splits;
@@ -404,7 +405,7 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     const int nt = std::min(256, tokens - t0);
     torch::Tensor xs = x.narrow(0, t0, nt);
     const int n_pad = (nt + 15) / 16 * 16;
-    const OprojForm form = oproj_form(hidden, K, n_pad, splits, true, helix::device_sm_count());
+    const OprojForm form = oproj_form(hidden, K, nt, splits, true, helix::device_sm_count());
     const helix::OprojSplitPlan plan = form.plan;
     const int sp = form.splits;
     ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024,
@@ -576,7 +577,7 @@ int gqa_launches(int B, int Hkv, int max_seq_len, int sm_count) {
 int oproj_launches(int tokens, int hidden, int K, bool packed, int sm_count) {
   int n = 0;
   for (int t0 = 0; t0 < tokens; t0 += 256)
-    n += oproj_form(hidden, K, (std::min(256, tokens - t0) + 15) / 16 * 16, 0, packed, sm_count).launches();
+    n += oproj_form(hidden, K, std::min(256, tokens - t0), 0, packed, sm_count).launches();
   return n;
 }
 

@@ -54,7 +54,7 @@ cudaError_t launch_oproj_streamk(const OprojParams& p, bool pdl, cudaStream_t st
 struct OprojSplitPlan {
   int slabs, splits;     // slabs 0: the plain kernel is the better one
 };
-OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int n_pad, int sm_count);
+OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int tokens, int sm_count);
 cudaError_t launch_oproj_split(const OprojParams& p, int slabs, bool pdl, cudaStream_t stream);
 
 }  // namespace helix

@@ -264,11 +264,10 @@ __global__ void __launch_bounds__(kSkThreads, 1) oproj_streamk_kernel(const __gr
 // oproj_split_fold_kernel sums them with all SMs.  oproj_pick_split_plan says which form a call takes.
 // Measured (packed weights, launches back to back in a graph, plain kernel -> this one): hidden 7168, K 8192, 200 tokens
 // 59.3 -> 40.5 us, 64 tokens 34.6 -> 29.1; hidden 2048, K 8192, 64 tokens 32.6 -> 15.5; hidden 4096, K 4096, 32 tokens
-// 17.6 -> 13.7.  Below 32 tokens and with at most two splits the two are level, and the plain kernel is one launch.
+// 17.6 -> 13.7.
 // kSlabs * 4 warps: warp 0 feeds the ring (`atoms` 64-wide K atoms per stage), warp 1 issues the MMAs, and each group of
 // four warps reads one slab's accumulator out.
 constexpr int kSplitMaxStages = 8;
-constexpr int kSplitMinTokens = 32;
 
 __host__ __device__ __forceinline__ int split_atom_bytes(int slabs, int n_pad) { return (slabs * kBM + n_pad) * kAtomK * 2; }
 
@@ -534,12 +533,20 @@ cudaError_t launch_oproj_streamk(const OprojParams& p, bool pdl, cudaStream_t st
 
 // A call's form is the cheapest of {one, two slabs} x K splits that fit the SMs at once, by what bounds the parts: a CTA
 // takes in its share of W and all of x for its K range at 58 GB/s; W arrives at 6 TB/s altogether; partials cost a
-// launch (3 us) and 0.25 us per MB.  The plain kernel (no second launch, four atoms per copy) keeps the calls that
-// it serves without a split, or with few tokens and no more than two.
-OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int n_pad, int sm_count) {
+// launch (5 us) and 0.25 us per MB.  The plain kernel (no second launch, four atoms per copy) keeps
+//   * up to 16 tokens with at most two K splits, where the two are level;
+//   * up to 8 tokens (its fold's step) from 3072 rows on: 5120 x 5120, 1 token 13.2 us against 14.6, 4096 x 4096 11.0 / 11.6;
+//     at 2048 rows and fewer the split form is level or ahead (1024 x 4096 10.3 against 9.1), and from 9 tokens on
+//     (4096 x 4096 14.1 / 13.6);
+//   * calls without a split that already fill three quarters of the SMs: 16384 x 5120, 128 tokens 39 us against 45.  With
+//     K of 16384 and more the partials no longer weigh as much (64 tokens 95 against 88).
+// With 3 us for the launch instead of 5 it lost 10240 x 2048 (32 tokens 14 us against 16) and 5120 x 1024 (64 tokens 10 / 11).
+OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int tokens, int sm_count) {
   OprojSplitPlan best{0, 0};
-  const int plain = oproj_pick_splits(hidden, K, sm_count);
-  if (n_pad < kSplitMinTokens && plain <= 2) return best;
+  const int n_pad = (tokens + 15) / 16 * 16, plain = oproj_pick_splits(hidden, K, sm_count);
+  if (tokens <= 16 && plain <= 2) return best;
+  if (tokens <= 8 && hidden > 2048) return best;
+  if (plain == 1 && hidden / kBM * 4 >= sm_count * 3 && K < 16384) return best;
   float best_us = 1e30f;
   const int n_atoms = K / kAtomK;
   for (int slabs = 1; slabs <= 2; ++slabs) {
@@ -548,7 +555,7 @@ OprojSplitPlan oproj_pick_split_plan(int hidden, int K, int n_pad, int sm_count)
     for (int splits = 1; splits <= most; ++splits) {
       const float in = (float)((n_atoms + splits - 1) / splits) * split_atom_bytes(slabs, n_pad) / 58e3f;
       const float w = (float)hidden * K * 2 / 6e6f * std::max(1.f, (float)sm_count * 0.75f / (groups * splits));
-      const float us = std::max(in, w) + (splits > 1 ? 3.f + 0.25e-6f * splits * n_pad * hidden * 4 : 0.f);
+      const float us = std::max(in, w) + (splits > 1 ? 5.f + 0.25e-6f * splits * n_pad * hidden * 4 : 0.f);
       if (us < best_us) best_us = us, best = OprojSplitPlan{slabs, splits};
     }
   }

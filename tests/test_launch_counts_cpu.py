@@ -23,3 +23,16 @@ def test_kernels_per_step_counts_every_launch(native_built):
     assert stack.kernels_per_step() == cfg.n_layers * 4
     stack.fuse_oproj = True
     assert stack.kernels_per_step() == cfg.n_layers * 3
+
+
+def test_oproj_keeps_one_launch_where_the_split_kernels_are_slower(native_built):
+    from helix_a2a_b200.ops._ext import ext
+    one = lambda hidden, K, tokens: ext().oproj_launches(tokens, hidden, K, True, 148) == 1   # noqa: E731
+    for hidden, K in ((3072, 4096), (4096, 4096), (5120, 5120), (6144, 4096), (8192, 8192)):
+        assert one(hidden, K, 1) and one(hidden, K, 8)
+    assert not one(1024, 4096, 1) and not one(2048, 8192, 8)              # few slabs: finer splits pay from the first token
+    assert not one(4096, 4096, 9) and not one(5120, 5120, 9) and one(8192, 8192, 16)
+    # no split to begin with: the second launch has to earn itself
+    for hidden, K, tokens in ((10240, 2048, 32), (5120, 1024, 64), (16384, 5120, 128), (16384, 8192, 256), (4096, 1024, 48)):
+        assert one(hidden, K, tokens), (hidden, K, tokens)
+    assert not one(10240, 8192, 32) and not one(16384, 16384, 64) and not one(1024, 2048, 17)
