@@ -122,11 +122,13 @@ def test_oproj_matches_fp32_matmul(built, monkeypatch, tokens, hidden, K, splits
 
 
 @pytest.mark.parametrize("hidden,K,splits,tokens", [(512, 256, 2, 300), (1024, 2048, 4, 300), (512, 256, 2, 17),
-                                                    (8192, 1024, 0, 8), (512, 256, -1, 300), (1024, 8192, 3, 300)])
+                                                    (8192, 1024, 0, 8), (512, 256, -1, 300), (1024, 8192, 3, 300),
+                                                    (2048, 4096, 0, 300), (1024, 8192, 0, 40), (4096, 2048, 0, 256)])
 def test_oproj_back_to_back_under_programmatic_launch(built, monkeypatch, hidden, K, splits, tokens):
     """Launches chained by programmatic dependent launch share the split-K scratch: a launch (a 256-token slice of a
     larger call, or the next call) must not touch it before the previous one is done, not even from a CTA that has
-    no k-block of its own (512 x 256 in two splits with one 256-wide stage: the second split is empty)."""
+    no k-block of its own (512 x 256 in two splits with one 256-wide stage: the second split is empty).  The last three
+    sizes run as split kernel and sum of its partials."""
     from helix_a2a_b200.ops.oproj import oproj, check_compute_status
     monkeypatch.setenv("HELIX_A2A_ENABLE_PDL", "1")
     monkeypatch.setenv("HELIX_A2A_OPROJ_LIBRARY", "0")
@@ -203,7 +205,7 @@ def _mla_case(seq_lens, page=16, seed=0):
     return qn, qp, ckv, scales, kpe, bt, torch.tensor(seq_lens, dtype=torch.int32, device="cuda")
 
 
-@pytest.mark.parametrize("variant", ["lockstep", "ws"])
+@pytest.mark.parametrize("variant", ["lockstep", "ws", "pair"])
 def test_mla_fp8_dequant_covers_every_e4m3_value(built, monkeypatch, variant):
     monkeypatch.setenv("HELIX_A2A_MLA_VARIANT", variant)
     """The kernels decode e4m3 with integer bit moves and bf16 multiplies: check all 254 finite byte values
@@ -236,7 +238,7 @@ def test_mla_fp8_dequant_covers_every_e4m3_value(built, monkeypatch, variant):
 
 @pytest.mark.parametrize("seq_lens,ctas", [([32], 1), ([100, 7, 64], 1), ([1000, 333], 3), ([4096, 2000, 17, 0], 0),
                                            ([700] * 5, 7)])
-@pytest.mark.parametrize("variant", ["lockstep", "ws"])
+@pytest.mark.parametrize("variant", ["lockstep", "ws", "pair"])
 def test_mla_fp8_decode_matches_fp32_reference(built, monkeypatch, seq_lens, ctas, variant):
     import math
     monkeypatch.setenv("HELIX_A2A_MLA_VARIANT", variant)

@@ -18,12 +18,14 @@ def _case(lens, hkv, group, page, layout, seed):
     return q, k, v, bt, torch.tensor(lens, dtype=torch.int32, device="cuda")
 
 
-# around one 16-token block, around the longest unsplit sequence (512 tokens), empty sequences, few and many pairs,
-# groups of one to eight heads; splits = 0 leaves the form to the library, the others force shares and the fold
+# around one 16-token block, empty sequences, few and many pairs, groups of one to eight heads; both sides of the longest
+# unsplit sequence on 148 SMs: 41 blocks (656 tokens) with 8 pairs, 96 blocks (1536 tokens) from 173 pairs on; splits = 0 leaves
+# the form to the library, the others force shares and the fold
 @pytest.mark.parametrize("lens,hkv,group,page,layout", [
     ([1], 1, 1, 16, "HND"), ([15, 16, 17, 0], 8, 8, 16, "NHD"), ([300], 8, 8, 16, "HND"), ([511, 512, 64], 2, 4, 32, "NHD"),
     ([513, 3], 8, 3, 16, "HND"), ([100] * 40 + [0, 1], 8, 8, 64, "HND"), ([2000, 0, 90, 7000], 4, 8, 16, "HND"),
-    ([40, 600] * 150, 2, 8, 16, "HND"), ([20000], 8, 8, 16, "NHD")])
+    ([40, 600] * 150, 2, 8, 16, "HND"), ([20000], 8, 8, 16, "NHD"), ([656], 8, 8, 16, "HND"), ([657], 8, 8, 16, "HND"),
+    ([1536, 5, 900, 0] * 25, 4, 2, 16, "HND"), ([1537, 5, 900, 0] * 25, 4, 2, 16, "NHD")])
 def test_forms_agree_with_the_oracle(native_built, lens, hkv, group, page, layout):
     from helix_a2a_b200.ops import attention, reference_math as rm
     from helix_a2a_b200.ops.oproj import check_compute_status

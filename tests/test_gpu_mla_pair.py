@@ -47,9 +47,10 @@ def _check(seq_lens, page, ctas, scale, base2=False, std=0.5, poison=False):
         # Dequantised values carry two bf16 roundings (scale, product), probabilities one, the result one: 4 x 2^-9 of
         # values that are at most about 4.5.  A score is off by at most 2^-8 of the sum of its four blocks' |q . k|, each
         # 0.5 * sqrt(128) / sqrt(192) = 0.41 in the standard deviation and under three of them: 2^-8 * 4 * 3 * 0.41 = 0.019.
-        # That is also the bound of the LSE (reached with one token only, longer sequences average it out).
+        # That is also the bound of the LSE with a few tokens.  From 64 on their errors, which have either sign, average
+        # out to less than a quarter of it: 5e-3, where a systematic error of the scores would show.
         assert (o[b].float() - o_ref[0]).abs().max() < 3e-2, (b, n)
-        assert (lse[b] - l_ref[0]).abs().max() < 1.9e-2 * (1.45 if base2 else 1), (b, n)
+        assert (lse[b] - l_ref[0]).abs().max() < (1.9e-2 if n < 64 else 5e-3) * (1.45 if base2 else 1), (b, n)
 
 
 # edges of the 64-token tile and of the 16-token unit, one to several tiles a piece, more sequences than clusters, empty
