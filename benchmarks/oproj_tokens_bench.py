@@ -4,7 +4,8 @@
 
     python benchmarks/oproj_tokens_bench.py [--iters 20]
 
-Rotating weight buffers larger than L2, CUDA events, >= 3 warm-ups; one JSON line per point.
+Rotating weight buffers larger than L2, CUDA events, >= 3 warm-ups; one JSON line per point.  Programmatic launch is on, as in
+the decode chain, so consecutive launches overlap; HELIX_A2A_ENABLE_PDL=0 times the launches one after the other.
 """
 import argparse
 import json
@@ -37,7 +38,7 @@ def main():
             us = time_rotating([(lambda l=l: oproj(x, wp[l])) for l in range(nl)], args.iters)
             us_ref = time_rotating([(lambda l=l: torch.nn.functional.linear(x, ws[l])) for l in range(nl)], args.iters)
             nbytes = hidden * K * 2 + T * K * 2 + T * hidden * 2
-            print(json.dumps({"kernel": "oproj (packed weights)", "cp": cp, "K": K, "tokens": T, "us": us,
+            print(json.dumps({"kernel": "oproj (packed weights)", "programmatic_launch": os.environ["HELIX_A2A_ENABLE_PDL"] == "1", "cp": cp, "K": K, "tokens": T, "us": us,
                               "torch_linear_us": us_ref, "frac_of_%s_hbm" % src: nbytes / us / 1e3 / hbm,
                               "tflops": 2 * T * K * hidden / us / 1e6}), flush=True)
             check_compute_status(x)

@@ -5,6 +5,7 @@
     python benchmarks/profile_case.py oproj     # o_proj, 8 tokens, K=8192, hidden 8192 (134 MB of W)
     python benchmarks/profile_case.py exchange  # fused exchange+combine, 4 ranks played by one launch
     python benchmarks/profile_case.py mla       # MLA fp8 decode, B=8, 16K tokens per sequence
+    python benchmarks/profile_case.py mla_64k   # the same with 64K tokens per sequence (344 MB of cache, larger than L2)
     python benchmarks/profile_case.py fused     # one-kernel exchange+combine+o_proj, 8 ranks played by one launch
     python benchmarks/profile_case.py fused_rows  # the same with 64 tokens (slabs of a head group share the rows)
     python benchmarks/profile_case.py streamk   # stream-K o_proj, 8 tokens, K=8192, hidden 8192
@@ -62,10 +63,10 @@ def main():
         w = (torch.randn(cp, hidden, (H // cp) * D, device="cuda") * 0.05).bfloat16()
         for _ in range(launches):
             ops().alltoall_combine_oproj(outs, lses, w, ws, 0, cp, False, True, 0)
-    elif which == "mla":
+    elif which in ("mla", "mla_64k"):
         import math
         from helix_a2a_b200.ops import attention, reference_math as rm
-        B, ctx, page = 8, 16384, 16
+        B, ctx, page = 8, (16384 if which == "mla" else 65536), 16
         pages = B * ctx // page
         bt = torch.randperm(pages).int().view(B, -1).cuda()
         sl = torch.full((B,), ctx, dtype=torch.int32, device="cuda")

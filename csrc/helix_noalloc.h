@@ -9,15 +9,14 @@
 // device memory through its own pool forbids libraries from calling the CUDA allocator behind its
 // back; and a plain C / C++ / Rust host that links this library without PyTorch has no caching
 // allocator to lean on at all.  Such callers own the inputs and outputs already.  What they cannot
-// supply is the kernel's private scratch (per-CTA partial results and arrival counters of the
-// split-KV merge), so here that scratch lives inside the library image.
+// supply is the kernel's private scratch (per-CTA partial results of the split-KV merge), so here
+// that scratch lives inside the library image.
 //
 // The scratch is ONE file-scope device array of fixed size (about 10.6 MB, see the limits below).
 // Every GPU that loads the library carries it from load until the process ends.  All eager calls on
 // a device share one half of it and all calls captured into CUDA graphs the other, and it keeps
-// whatever the previous call left behind: the entry point clears the parts that must start at zero
-// (arrival counters, error word) on the caller's stream before each launch.  Threads may call on one
-// stream.  Because the array is shared, two calls whose kernels may overlap on the same GPU (for
+// whatever the previous call left behind: the entry point clears the error word on the caller's
+// stream before each launch.  Threads may call on one stream.  Because the array is shared, two calls whose kernels may overlap on the same GPU (for
 // instance on different streams) race on it; callers must order such calls themselves.
 //
 // The first call on each device performs a one-time set-up (it resolves the device address of the
@@ -33,8 +32,8 @@
 extern "C" {
 #endif
 
-// Limits of the built-in scratch.  Larger problems are rejected with kHelixNoAllocTooLarge.
-#define HELIX_NOALLOC_MAX_PAIRS 4096   /* batch * kv_heads */
+// Limits of this entry point.  Larger problems are rejected with kHelixNoAllocTooLarge.
+#define HELIX_NOALLOC_MAX_PAIRS 4096   /* batch * kv_heads: part of the contract, the scratch does not depend on it */
 #define HELIX_NOALLOC_MAX_CTAS 640     /* CTAs of one launch (the library picks at most 2 per SM) */
 
 enum HelixNoAllocStatus {

@@ -20,15 +20,13 @@ namespace {
 // A set:
 //   [0, kPartO)                    partial outputs   [MAX_CTAS][2][8][128] fp32
 //   [kPartO, kPartO + kPartL)      partial LSEs      [MAX_CTAS][2][8]      fp32, and what each CTA notes for the fold (16 bytes)
-//   then                           arrival counters  [MAX_PAIRS]           int32   (must be zero at launch)
 // Error word: int32 (+ padding), must be zero at launch.
 // A call is up to two launches that meet in its set, so it holds the device's lock from the first to the last (threads
 // may share a stream), and a graph that one thread replays between the launches of another's eager call finds its own set.
 constexpr size_t kPartO = (size_t)HELIX_NOALLOC_MAX_CTAS * 2 * 8 * 128 * sizeof(float);
 constexpr size_t kPartL = (size_t)HELIX_NOALLOC_MAX_CTAS * (2 * 8 + 4) * sizeof(float);
-constexpr size_t kCounters = (size_t)HELIX_NOALLOC_MAX_PAIRS * sizeof(int);
 constexpr size_t kErr = 256;
-constexpr size_t kSetBytes = kPartO + kPartL + kCounters, kErrAt = 2 * kSetBytes;
+constexpr size_t kSetBytes = kPartO + kPartL, kErrAt = 2 * kSetBytes;
 constexpr size_t kScratchBytes = kErrAt + kErr;
 static_assert(kSetBytes % 256 == 0, "both sets are aligned alike");
 static_assert(HELIX_NOALLOC_MAX_CTAS <= helix::kGqaMaxCtas, "the kernel's grid bound sizes the piece slots");
@@ -111,7 +109,7 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
     return kHelixNoAllocBadArgument;
   }
   if ((int64_t)batch * kv_heads > HELIX_NOALLOC_MAX_PAIRS) {
-    snprintf(g_err, sizeof(g_err), "batch * kv_heads = %lld exceeds the built-in scratch (max %d)",
+    snprintf(g_err, sizeof(g_err), "batch * kv_heads = %lld exceeds the limit of this entry point (%d)",
              (long long)batch * kv_heads, HELIX_NOALLOC_MAX_PAIRS);
     return kHelixNoAllocTooLarge;
   }
@@ -142,7 +140,7 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
   p.lse = lse;
   p.part_o = reinterpret_cast<float*>(base);
   p.part_lse = reinterpret_cast<float*>(base + kPartO);
-  p.counters = reinterpret_cast<int*>(base + kPartO + kPartL);
+  p.counters = nullptr;      // only the pools of the dynamic tail count anything
   p.error_flag = reinterpret_cast<int*>(st->base + kErrAt);
   p.trace = nullptr;
   p.B = batch;
@@ -159,10 +157,8 @@ extern "C" __attribute__((visibility("default"))) int helix_gqa_decode_noalloc(
   p.scale = scale;
   p.lse_base2 = lse_base2 ? 1 : 0;
   p.timeout_ns = 2000000000ull;
-  // the array keeps the previous call's contents: counters and the error word must start at zero
-  cudaError_t e = cudaMemsetAsync(p.counters, 0, (size_t)batch * kv_heads * sizeof(int), s);
-  if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counters)");
-  e = cudaMemsetAsync(p.error_flag, 0, sizeof(int), s);
+  // the array keeps the previous call's contents: the error word must start at zero
+  cudaError_t e = cudaMemsetAsync(p.error_flag, 0, sizeof(int), s);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(error word)");
   e = helix::launch_gqa_decode(p, false, s);
   if (e != cudaSuccess) return fail_cuda(e, "kernel launch");
