@@ -1,6 +1,5 @@
 // Torch bindings of the compute kernels (decode attention, o_proj GEMM).
 #include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -50,8 +49,12 @@ struct Scratch {
   torch::Tensor trace;         // int64 [rows * 8], only with one of the *_TRACE / *_PROF variables set
   std::vector<torch::Tensor> retired;
 };
-std::mutex g_mu;
-std::map<int, Scratch> g_scratch;
+std::mutex g_mu;                 // tensor-map cache
+Scratch g_scratch[64];           // by device
+
+void check_cuda(cudaError_t e, const char* what) {
+  TORCH_CHECK(e == cudaSuccess, "helix: ", what, " failed: ", cudaGetErrorString(e));
+}
 
 struct ScratchUse {
   Scratch& dev;
@@ -59,30 +62,34 @@ struct ScratchUse {
   std::unique_lock<std::mutex> held;
 };
 
-ScratchUse scratch_for(const torch::Device& dev, int64_t counters, int64_t part_a_floats, int64_t part_b_floats) {
-  Scratch* entry;
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    entry = &g_scratch[dev.index()];
-  }
-  Scratch& s = *entry;
+// used: the call's kernels touch counters or partials.  Those that do not (unsplit attention, o_proj without a K split) are
+// spared the question whether the stream is being captured, once the sets are there.
+ScratchUse scratch_for(const torch::Device& dev, bool used, int64_t counters, int64_t part_a_floats, int64_t part_b_floats) {
+  TORCH_CHECK(dev.index() >= 0 && dev.index() < 64, "device index out of range");
+  Scratch& s = g_scratch[dev.index()];
   std::unique_lock<std::mutex> held(s.launching);
-  auto iopt = torch::TensorOptions().dtype(torch::kInt32).device(dev);
-  auto fopt = torch::TensorOptions().dtype(torch::kFloat32).device(dev);
-  auto grow = [&](torch::Tensor& t, int64_t need, int64_t floor, const torch::TensorOptions& opt, bool zero) {
+  auto grow = [&](torch::Tensor& t, int64_t need, int64_t floor, torch::ScalarType type, bool zero) {
     if (t.defined() && t.numel() >= need) return;
     if (t.defined()) s.retired.push_back(t);
+    const auto opt = torch::TensorOptions().dtype(type).device(dev);
     const int64_t n = std::max<int64_t>(need + need / 4, floor);     // head-room: regrowing is rare
     t = zero ? torch::zeros({n}, opt) : torch::empty({n}, opt);
   };
-  if (!s.error_flag.defined()) s.error_flag = torch::zeros({1}, iopt);
-  const bool captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  auto holds = [](const torch::Tensor& t, int64_t need) { return t.defined() && t.numel() >= need; };
+  auto ready = [&](const Scratch::Set& t) {
+    return holds(t.counters, counters) && holds(t.part_a, part_a_floats) && holds(t.part_b, part_b_floats);
+  };
+  grow(s.error_flag, 1, 1, torch::kInt32, true);
+  if (!used && ready(s.sets[0]) && ready(s.sets[1])) return {s, s.sets[0], std::move(held)};
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  check_cuda(cudaStreamIsCapturing(at::cuda::getCurrentCUDAStream(dev.index()), &status), "stream capture query");
+  const bool captured = status != cudaStreamCaptureStatusNone;
   // An eager call grows both sets: what is captured after a warm-up finds its own ready, its counters zeroed by a memset
   // that has run and is not part of the graph.
   for (int i = captured ? 1 : 0; i < 2; ++i) {
-    grow(s.sets[i].counters, counters, 16384, iopt, true);
-    grow(s.sets[i].part_a, part_a_floats, 1, fopt, false);
-    grow(s.sets[i].part_b, part_b_floats, 1, fopt, false);
+    grow(s.sets[i].counters, counters, 16384, torch::kInt32, true);
+    grow(s.sets[i].part_a, part_a_floats, 1, torch::kFloat32, false);
+    grow(s.sets[i].part_b, part_b_floats, 1, torch::kFloat32, false);
   }
   return {s, s.sets[captured ? 1 : 0], std::move(held)};
 }
@@ -99,10 +106,6 @@ unsigned long long* trace_for(Scratch& s, const torch::Device& dev, int64_t rows
 int env_int(const char* name, int dflt) {
   const char* v = std::getenv(name);
   return (v && *v) ? std::atoi(v) : dflt;
-}
-
-void check_cuda(cudaError_t e, const char* what) {
-  TORCH_CHECK(e == cudaSuccess, "helix: ", what, " failed: ", cudaGetErrorString(e));
 }
 
 // ---- tensor-map cache --------------------------------------------------------------------------
@@ -180,12 +183,13 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   int sp = splits > 0 ? (int)std::min<int64_t>((int64_t)B * Hkv * splits, helix::kGqaMaxCtas)
                       : helix::gqa_pick_ctas(B, Hkv, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
   sp = std::max(sp, 1);
+  const bool whole = splits <= 0 && helix::gqa_whole_pairs(B, Hkv, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
   torch::Tensor o = torch::empty({B, Hq, 128}, q.options());
   torch::Tensor lse = torch::empty({B, Hq}, q.options().dtype(torch::kFloat32));
   if (B == 0) return std::make_tuple(o, lse);
   const int max_helper = helix::kGqaMaxHelper;
   // the o_proj counters sit in the last hidden / 128 ints of the same tensor: leave them room
-  ScratchUse sc = scratch_for(q.device(), (int64_t)helix::gqa_counter_ints(B * Hkv, max_helper) + 2048,
+  ScratchUse sc = scratch_for(q.device(), !whole, (int64_t)helix::gqa_counter_ints(B * Hkv, max_helper) + 2048,
                             (int64_t)helix::gqa_part_o_floats(sp, max_helper),
                             (int64_t)helix::gqa_part_lse_floats(sp, max_helper));
   helix::GqaDecodeParams p{};
@@ -204,7 +208,7 @@ std::tuple<torch::Tensor, torch::Tensor> gqa_decode(torch::Tensor q, torch::Tens
   p.counters = sc.set.counters.data_ptr<int32_t>();
   p.error_flag = sc.dev.error_flag.data_ptr<int32_t>();
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.page_size = page; p.ctas = sp;
-  p.whole = splits <= 0 && helix::gqa_whole_pairs(B, Hkv, (int)std::max<int64_t>(max_seq_len, 1), helix::device_sm_count());
+  p.whole = whole;
   // HELIX_A2A_ATTN_DYN_PCT / HELIX_A2A_ATTN_DYN_CHUNK: share of every long pair that is handed out dynamically
   // (0 = fixed shares only) and the chunk size in 16-token blocks; unset = the library's choice
   helix::gqa_plan_dynamic(&p, (int)std::max<int64_t>(max_seq_len, 1), max_helper, env_int("HELIX_A2A_ATTN_DYN_PCT", -1),
@@ -278,7 +282,7 @@ std::tuple<torch::Tensor, torch::Tensor> mla_decode(torch::Tensor q_nope, torch:
            : variant == 2 ? helix::mla_pair_pick_ctas(B, longest, helix::device_sm_count())
                           : helix::mla_pick_ctas(B, longest, helix::device_sm_count());
   if (variant == 2) nc = std::max(nc / 2 * 2, 2);
-  ScratchUse sc = scratch_for(q_nope.device(), (int64_t)B + 1024, (int64_t)helix::mla_part_o_floats(nc),
+  ScratchUse sc = scratch_for(q_nope.device(), true, (int64_t)B + 1024, (int64_t)helix::mla_part_o_floats(nc),
                             (int64_t)helix::mla_part_lse_floats(nc));
   helix::MlaDecodeParams p{};
   p.q_nope = reinterpret_cast<const __nv_bfloat16*>(q_nope.data_ptr());
@@ -357,7 +361,7 @@ torch::Tensor oproj(torch::Tensor x, torch::Tensor w, int64_t splits) {
     const int sk_ctas = (int)std::min<int64_t>(sms, (int64_t)(hidden / 128) * ((K + bk - 1) / bk));
     const int64_t part_floats = streamk ? (int64_t)helix::oproj_streamk_partial_floats(sk_ctas, n_pad)
                                         : (sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0);
-    ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024, part_floats, 0);
+    ScratchUse sc = scratch_for(x.device(), part_floats > 0, hidden / 128 + 1024, part_floats, 0);
     helix::OprojParams p{};
     p.w_map = mat_map(w, 128);
     p.x_map = mat_map(xs, n_pad);
@@ -408,7 +412,7 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
     const OprojForm form = oproj_form(hidden, K, nt, splits, true, helix::device_sm_count());
     const helix::OprojSplitPlan plan = form.plan;
     const int sp = form.splits;
-    ScratchUse sc = scratch_for(x.device(), hidden / 128 + 1024,
+    ScratchUse sc = scratch_for(x.device(), sp > 1, hidden / 128 + 1024,
                               sp > 1 ? (int64_t)helix::oproj_partial_bytes(hidden, sp, n_pad) / 4 : 0, 0);
     helix::OprojParams p{};
     p.x_map = mat_map(xs, n_pad);
@@ -431,7 +435,7 @@ torch::Tensor oproj_packed(torch::Tensor x, torch::Tensor packed, int64_t hidden
 }
 
 torch::Tensor attn_trace(torch::Tensor like) {
-  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  ScratchUse sc = scratch_for(like.device(), false, 1, 0, 0);
   TORCH_CHECK(sc.dev.trace.defined(), "no trace recorded: set HELIX_A2A_ATTN_TRACE=1 (or HELIX_A2A_OPROJ_TRACE=1)");
   return sc.dev.trace.clone();
 }
@@ -488,7 +492,7 @@ std::tuple<torch::Tensor, torch::Tensor> fused_impl(torch::Tensor attn_out, torc
   torch::Tensor y = torch::empty(ys, attn_out.options());
   const int n_pad = (int)((B + 15) / 16 * 16);
   const int64_t part_floats = splits > 1 ? (int64_t)helix::oproj_partial_bytes((int)hidden, splits, n_pad) / 4 * ranks : 0;
-  ScratchUse sc = scratch_for(attn_out.device(), (hidden / 128 + helix::fused_aux_ints((int)hidden)) * ranks + 1024, part_floats, 0);
+  ScratchUse sc = scratch_for(attn_out.device(), true, (hidden / 128 + helix::fused_aux_ints((int)hidden)) * ranks + 1024, part_floats, 0);
 
   helix::FusedParams fp{};
   helix::ExchangeParams& p = fp.ex;
@@ -582,12 +586,12 @@ int oproj_launches(int tokens, int hidden, int K, bool packed, int sm_count) {
 }
 
 int64_t read_error_flag(torch::Tensor like) {
-  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  ScratchUse sc = scratch_for(like.device(), false, 1, 0, 0);
   return sc.dev.error_flag.item<int>();
 }
 
 void clear_error_flag(torch::Tensor like) {
-  ScratchUse sc = scratch_for(like.device(), 1, 0, 0);
+  ScratchUse sc = scratch_for(like.device(), false, 1, 0, 0);
   sc.dev.error_flag.zero_();
   for (Scratch::Set& set : sc.dev.sets) set.counters.zero_();
 }
