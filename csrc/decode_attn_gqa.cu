@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 2) gqa_decode_kernel(const __grid_co
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kWarps][kStages];
   __shared__ float s_m[kWarps][8], s_l[kWarps][8];
-  __shared__ int s_flag;                         // CTA-wide broadcast word (last arrival, scan result, list length)
+  __shared__ int s_flag;                         // first pool with chunks left, while the pools are being probed
   __shared__ int s_draw[2];                      // chunk drawn ahead by thread 0 (two slots, used alternately)
   __shared__ int s_scan;                         // chunk drawn while probing the other pools
   __shared__ int s_nb[kGqaSeqTable];             // KV blocks of each sequence
@@ -971,7 +971,8 @@ __global__ void __launch_bounds__(kFoldThreads) gqa_fold_starts_kernel(const __g
 
 // Number of CTAs for a launch: two per SM, but never so many that a CTA streams fewer than 8 blocks (two per warp).
 // With 32 blocks as the limit one sequence of 4000 tokens (8 kv heads) took 19.6 us and four of up to 1000 took
-// 21.6 us; with about 128 CTAs each 17.3 and 15.9 us.
+// 21.6 us; with about 128 CTAs each 17.3 and 15.9 us.  Not the best choice everywhere: one sequence of 700 tokens takes 14.5 us
+// with the 44 CTAs it gets and 10.6 with 296, and 8 x 1536 tokens take 21.5 where 192 CTAs of 32 blocks took 19.
 int gqa_pick_ctas(int B, int Hkv, int max_seq_len, int sm_count) {
   const long long blocks = (long long)std::max(B, 1) * Hkv * std::max((max_seq_len + kBlockTok - 1) / kBlockTok, 1);
   long long ctas = std::min<long long>(2LL * sm_count, std::max<long long>(blocks / kMinShare, 1));

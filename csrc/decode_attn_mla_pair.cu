@@ -22,14 +22,11 @@
 // the others), so that one group's way to the peer and back is covered by the other's arithmetic; warps 12..19
 // dequantise, fed by register prefetch one tile ahead.  The MMA queue runs Q K^T two tiles ahead of P V.
 // Pieces of a sequence are merged by a second small kernel (mla_pair_fold_kernel) with all SMs.
-// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 419 us, 16 ragged
+// Measured against the warp-specialised single-CTA kernel (B200, one call): 32 x 32768 tokens 661 -> 416 us, 16 ragged
 // sequences up to 17000 tokens 252 -> 84 us (a last-CTA fold read all pieces through one SM), 2 x 1500 tokens 121 -> 26 us.
-// On the way there (32 x 32768): one softmax group whose threads exchanged all partial scores, 606 us with buffer
-// credits and 495 without; two groups 478; each CTA finishing half of the heads 445; MMAs issued under one convergent
-// elect with operands in uniform registers 430; one tile of prefetch instead of two, whose registers the softmax warps
-// put to better use, 419.  Lost: a third of the warps more (32 tokens a thread, 520); a second score
-// buffer with a quarter of Q in shared memory (446 against 445); a tile exchanged in two halves (461 against 445); the
-// next scores fetched before P goes out (573 against 393 in a graph: the registers spill).
+// Behind it by up to 1.4x: 128 sequences and more of one to four tiles each when the bound given for their lengths is far
+// larger (600 x 16 tokens 146 against 180 us), because a cluster takes them one after the other at ~18 us each; with
+// their real bound the single-CTA kernel takes 339.
 // Every wait is bounded; on expiry the error flag is raised, tensor memory is released and the kernel returns.
 #include "attention.h"
 

@@ -17,9 +17,12 @@ def oproj(x: torch.Tensor, w, *, splits: int = 0, library: Optional[bool] = None
     some idle), -1 forces the stream-K kernel, ``n >= 1`` forces the plain kernel with ``n`` K splits.
 
     The hand-written kernel is built for decode: few tokens, bound by streaming W once (swap-AB, one 128-row slab
-    of W per CTA, every CTA reads all of x).  With many tokens the product is compute-bound and every slab's CTA
-    re-reads x, and cuBLAS is faster (measured on B200 inside CUDA graphs, hidden 8192: level up to 8 tokens, 10-40 %
-    ahead at 32-64 tokens, 2x at 128).  So with ``splits=0`` and a plain weight matrix calls of 32 tokens or more go to
+    of W per CTA, every CTA reads all of x); above 16 tokens it splits K finely and sums the partials in a second
+    kernel.  Every slab's CTA re-reads x, so with many tokens cuBLAS is faster (measured on B200 inside CUDA graphs,
+    hidden 8192, K = 8192 / 4096 / 2048 / 1024, packed weights under programmatic launch against cuBLAS: 8 tokens
+    25.0 / 14.6 / 9.3 / 5.6 us against 23.8 / 13.4 / 7.8 / 5.6, 32 tokens 27.7 / 17.5 / 12.7 / 6.9 against
+    25.6 / 14.4 / 8.2 / 5.8, 128 tokens 35.8 / 22.8 / 16.7 / 11.0 against 25.7 / 14.1 / 8.6 / 6.3; launches that do not
+    overlap take about 3 us more).  So with ``splits=0`` and a plain weight matrix calls of 32 tokens or more go to
     ``torch.nn.functional.linear``; ``library=False`` (or ``HELIX_A2A_OPROJ_LIBRARY=0``) keeps the hand-written
     kernel for every size.  Packed weights always use the hand-written kernel (the plain matrix is not kept).
     """
