@@ -24,8 +24,8 @@ namespace {
 
 using namespace dev;
 
-template <bool COMBINE, bool BF16, int NIT>
-__global__ void __launch_bounds__(512, 1) helix_exchange_kernel(const __grid_constant__ ExchangeParams p) {
+template <bool COMBINE, bool BF16, int NIT, int CTAS_PER_SM>
+__global__ void __launch_bounds__(512, CTAS_PER_SM) helix_exchange_kernel(const __grid_constant__ ExchangeParams p) {
   extern __shared__ __align__(16) uint8_t dyn_smem[];
   __shared__ Control ctl;
 
@@ -69,9 +69,9 @@ __global__ void __launch_bounds__(512, 1) helix_exchange_kernel(const __grid_con
 
 using KernelFn = void (*)(ExchangeParams);
 
-template <int NIT>
+template <int NIT, int CTAS_PER_SM>
 KernelFn pick_combine(bool bf16) {
-  return bf16 ? (KernelFn)helix_exchange_kernel<true, true, NIT> : (KernelFn)helix_exchange_kernel<true, false, NIT>;
+  return bf16 ? (KernelFn)helix_exchange_kernel<true, true, NIT, CTAS_PER_SM> : (KernelFn)helix_exchange_kernel<true, false, NIT, CTAS_PER_SM>;
 }
 
 // kernel instance + compile-time iteration count for a call
@@ -81,16 +81,21 @@ struct Variant {
 };
 
 Variant pick_variant(const ExchangeParams& p, int iters) {
+  // A launch that plays several ranks shares the SMs between them, and a rank has a ring for every SM: its warps are too
+  // few to hide the latency of one message at a time, so messages of up to three iterations get the instance with half
+  // of the registers, two CTAs per SM.  Device time, cold L2: 8 ranks, 64 tokens, 64 heads of 128: 48.3 -> 23.1 us; 128 heads of 512:
+  // 8 ranks, 64 tokens 76.3 -> 66.2, 4 ranks, 32 tokens 24.3 -> 23.4, 2 ranks, 4 tokens 8.3 -> 7.5.
+  const bool shared = p.ranks_in_launch > 1;
   if (p.mode == kModeCombine) {
-    if (iters <= 1) return {pick_combine<1>(p.is_bf16), 1};
-    if (iters <= 2) return {pick_combine<2>(p.is_bf16), 2};
-    if (iters <= 3) return {pick_combine<3>(p.is_bf16), 3};
-    if (iters <= 5) return {pick_combine<5>(p.is_bf16), 5};
-    if (iters <= 9) return {pick_combine<9>(p.is_bf16), 9};
+    if (iters <= 1) return {shared ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1};
+    if (iters <= 2) return {shared ? pick_combine<2, 2>(p.is_bf16) : pick_combine<2, 1>(p.is_bf16), 2};
+    if (iters <= 3) return {shared ? pick_combine<3, 2>(p.is_bf16) : pick_combine<3, 1>(p.is_bf16), 3};
+    if (iters <= 5) return {pick_combine<5, 1>(p.is_bf16), 5};
+    if (iters <= 9) return {pick_combine<9, 1>(p.is_bf16), 9};
     return {nullptr, 0};
   }
-  if (iters <= 1) return {(KernelFn)helix_exchange_kernel<false, true, 1>, 1};
-  return {(KernelFn)helix_exchange_kernel<false, true, 3>, 3};  // larger messages go in slabs of 3
+  if (iters <= 1) return {(KernelFn)helix_exchange_kernel<false, true, 1, 1>, 1};
+  return {(KernelFn)helix_exchange_kernel<false, true, 3, 1>, 3};  // larger messages go in slabs of 3
 }
 
 size_t group_smem_bytes(int nit, int recv_warps, int group_warps) {
@@ -232,7 +237,15 @@ cudaError_t launch_exchange(ExchangeParams p, int channel_override, bool pdl, cu
   if (capacity <= 0) return cudaErrorLaunchOutOfResources;
   int cap_channels = capacity / p.ranks_in_launch;
   if (cap_channels < 1) return cudaErrorLaunchOutOfResources;
-  li.channels = std::min(li.channels, cap_channels);
+  if (li.channels > cap_channels) {
+    // fewer channels, more entries for each: the split of its warps is chosen again
+    li = plan_launch(p, cap_channels);
+    threads = 32 * (li.send_warps + li.recv_warps);
+    smem = p.mode == kModeCombine ? group_smem_bytes(var.nit, li.recv_warps, li.group_warps) : 0;
+    capacity = resident_ctas(var.fn, threads, smem);
+    if (capacity < p.ranks_in_launch) return cudaErrorLaunchOutOfResources;
+    li.channels = std::min(li.channels, capacity / p.ranks_in_launch);
+  }
 
   p.channels = li.channels;
   p.recv_warps = li.recv_warps;
