@@ -82,14 +82,17 @@ struct Variant {
 
 Variant pick_variant(const ExchangeParams& p, int iters) {
   // A launch that plays several ranks shares the SMs between them, and a rank has a ring for every SM: its warps are too
-  // few to hide the latency of one message at a time, so messages of up to three iterations get the instance with half
-  // of the registers, two CTAs per SM.  Device time, cold L2: 8 ranks, 64 tokens, 64 heads of 128: 48.3 -> 23.1 us; 128 heads of 512:
-  // 8 ranks, 64 tokens 76.3 -> 66.2, 4 ranks, 32 tokens 24.3 -> 23.4, 2 ranks, 4 tokens 8.3 -> 7.5.
-  const bool shared = p.ranks_in_launch > 1;
+  // few to hide the latency of one message at a time, so there is an instance with half of the registers, two CTAs per SM.
+  // Rows of 128 (one iteration) always take it; with longer ones it spills and pays from some 64 entries per channel on.
+  // One call, one CTA per SM -> two (the plan made again for the channels that fit in both), us: 64 heads of 128, 8 ranks, 32 / 128
+  // tokens 27.6 -> 16.3 / 54.1 -> 36.0; 128 heads of 512, 4 / 8 ranks, 128 tokens (110 entries a channel) 75.0 -> 64.8 / 140 -> 125,
+  // but 2 ranks, 32 tokens (28 a channel) 14.3 -> 16.6 and 8 ranks, 8 tokens 17.4 -> 21.0.
+  const int ranks = p.ranks_in_launch, per_channel = p.outer * p.inner / std::max(device_sm_count() / ranks, 1);
+  const bool dense = ranks > 1 && (iters <= 1 || per_channel >= 64);
   if (p.mode == kModeCombine) {
-    if (iters <= 1) return {shared ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1};
-    if (iters <= 2) return {shared ? pick_combine<2, 2>(p.is_bf16) : pick_combine<2, 1>(p.is_bf16), 2};
-    if (iters <= 3) return {shared ? pick_combine<3, 2>(p.is_bf16) : pick_combine<3, 1>(p.is_bf16), 3};
+    if (iters <= 1) return {dense ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1};
+    if (iters <= 2) return {dense ? pick_combine<2, 2>(p.is_bf16) : pick_combine<2, 1>(p.is_bf16), 2};
+    if (iters <= 3) return {dense ? pick_combine<3, 2>(p.is_bf16) : pick_combine<3, 1>(p.is_bf16), 3};
     if (iters <= 5) return {pick_combine<5, 1>(p.is_bf16), 5};
     if (iters <= 9) return {pick_combine<9, 1>(p.is_bf16), 9};
     return {nullptr, 0};
