@@ -20,7 +20,7 @@ from typing import Optional, Tuple
 import torch
 import torch.distributed as dist
 
-from .ops import reference_math as rm
+from .ops import _ext, reference_math as rm
 from .parallel import cpu_backend, workspace as ws_mod
 from .parallel.workspace import CpuWorkspace
 from .utils.tracing import check_written, nvtx_range
@@ -120,9 +120,8 @@ def alltoall(partial_o: torch.Tensor, softmax_stats: torch.Tensor, workspace: to
     """
     if isinstance(workspace, CpuWorkspace):
         return cpu_backend.alltoall(partial_o, softmax_stats, workspace._helix_group, cp_size)
-    from .ops._ext import ops
     with nvtx_range("helix.alltoall"):
-        ro, rs = ops().alltoall_helix_native(partial_o, softmax_stats, workspace, cp_rank, cp_size)
+        ro, rs = _ext.ops().alltoall_helix_native(partial_o, softmax_stats, workspace, cp_rank, cp_size)
     check_written(ro, "alltoall output")
     return ro, rs
 
@@ -157,11 +156,10 @@ def alltoall_combine(attn_out: torch.Tensor, lse: torch.Tensor, workspace: torch
     if cp_size == 1 and layout == "native" and lse.dim() == 2:
         # nothing to exchange or combine
         return (attn_out, lse) if return_lse else attn_out
-    from .ops._ext import ops
     with nvtx_range("helix.alltoall_combine"):
-        out, glse = ops().alltoall_combine(attn_out, lse, workspace, cp_rank, cp_size,
-                                           0 if layout == "native" else 1, return_lse, base2,
-                                           _STATS_MODES[stats_mode], False, 0, timeout_ms)
+        out, glse = _ext.ops().alltoall_combine(attn_out, lse, workspace, cp_rank, cp_size,
+                                                0 if layout == "native" else 1, return_lse, base2,
+                                                _STATS_MODES[stats_mode], False, 0, timeout_ms)
     check_written(out, "alltoall_combine output")
     return (out, glse) if return_lse else out
 
@@ -232,8 +230,9 @@ def lse_combine(outputs: torch.Tensor, lses: torch.Tensor, *, return_lse: bool =
         if return_lse:
             return res[0].to(outputs.dtype), res[1]
         return res.to(outputs.dtype)
-    from .ops._ext import ops
-    out, g = ops().lse_combine(outputs, lses.float(), 0 if layout == "NBHD" else -2, return_lse, base2)
+    if lses.dtype != torch.float32:
+        lses = lses.float()
+    out, g = _ext.ops().lse_combine(outputs, lses, 0 if layout == "NBHD" else -2, return_lse, base2)
     return (out, g) if return_lse else out
 
 

@@ -41,6 +41,20 @@ def available() -> bool:
         return False
 
 
+class _Ops:
+    """``torch.ops.helix_a2a_b200`` with every op resolved to its overload once: a call through the packet looks the
+    overload up again (about a microsecond of a call that takes seven)."""
+
+    def __getattr__(self, name):
+        op = getattr(torch.ops.helix_a2a_b200, name).default
+        setattr(self, name, op)
+        return op
+
+
+_ops = _Ops()
+
+
 def ops():
-    ext()
-    return torch.ops.helix_a2a_b200
+    if _mod is None:
+        ext()
+    return _ops

@@ -12,7 +12,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import reference_math as rm
+from . import _ext, reference_math as rm
 
 
 def gqa_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
@@ -36,10 +36,9 @@ def gqa_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bl
         vc = v_cache if layout == "HND" else v_cache.permute(0, 2, 1, 3)
         o, lse = rm.paged_decode_attention_reference(q, kc, vc, block_table, seq_lens, scale, lse_base2)
         return o.to(q.dtype), lse
-    from ._ext import ops
     if max_seq_len <= 0:
         max_seq_len = block_table.shape[1] * (k_cache.shape[2] if layout == "HND" else k_cache.shape[1])
-    return ops().gqa_decode(q, k_cache, v_cache, block_table, seq_lens, float(scale), lse_base2,
+    return _ext.ops().gqa_decode(q, k_cache, v_cache, block_table, seq_lens, float(scale), lse_base2,
                             layout == "HND", splits, max_seq_len, kv_stable)
 
 
@@ -70,8 +69,7 @@ def mla_decode(q_nope: torch.Tensor, q_pe: torch.Tensor, ckv_fp8: torch.Tensor, 
             outs.append(o)
             lses.append(l)
         return torch.cat(outs).to(q_nope.dtype), torch.cat(lses)
-    from ._ext import ops
     if max_seq_len <= 0:
         max_seq_len = block_table.shape[1] * ckv_fp8.shape[1]
-    return ops().mla_decode(q_nope, q_pe, ckv_fp8, scales, kpe, block_table, seq_lens, float(scale), lse_base2,
+    return _ext.ops().mla_decode(q_nope, q_pe, ckv_fp8, scales, kpe, block_table, seq_lens, float(scale), lse_base2,
                             ctas, max_seq_len)

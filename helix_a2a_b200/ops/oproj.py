@@ -9,6 +9,9 @@ from typing import Optional
 
 import torch
 
+from . import _ext
+from ..utils import env as _env
+
 
 def oproj(x: torch.Tensor, w, *, splits: int = 0, library: Optional[bool] = None) -> torch.Tensor:
     """``x [tokens, K]`` bf16, ``w [hidden, K]`` bf16 (``nn.Linear`` weight layout) -> bf16 ``[tokens, hidden]``.
@@ -29,23 +32,18 @@ def oproj(x: torch.Tensor, w, *, splits: int = 0, library: Optional[bool] = None
     if isinstance(w, PackedOprojWeight):
         if not x.is_cuda:
             return (x.float() @ unpack_weight(w).float().t()).to(x.dtype)
-        from ._ext import ops
-        return ops().oproj_packed(x, w.packed, w.hidden, w.K, max(splits, 0))
+        return _ext.ops().oproj_packed(x, w.packed, w.hidden, w.K, max(splits, 0))
     if not x.is_cuda:
         return (x.float() @ w.float().t()).to(x.dtype)
     if splits == 0 and library is not False and library_gemm_pays(x.shape[0], w.shape[1]):
         return torch.nn.functional.linear(x, w)
-    from ._ext import ops
-    return ops().oproj(x, w, splits)
+    return _ext.ops().oproj(x, w, splits)
 
 
 def library_gemm_pays(tokens: int, K: int) -> bool:
     """The measured crossover between the decode kernel and cuBLAS (see :func:`oproj`)."""
-    from ..utils import env as _env
-    if not _env.oproj_library():
-        return False
     del K          # the crossover does not depend on it: 32 tokens at K = 1024 ... 8192
-    return tokens >= 32
+    return tokens >= 32 and _env.oproj_library()
 
 
 class PackedOprojWeight:
@@ -96,7 +94,7 @@ def unpack_weight(pw: PackedOprojWeight) -> torch.Tensor:
 
 def check_compute_status(like: torch.Tensor) -> None:
     """Raise if an attention / GEMM kernel gave up on a bounded wait since the last check."""
-    from ._ext import ops
+    ops = _ext.ops
     code = int(ops().read_error_flag(like))
     if code != 0:
         ops().clear_error_flag(like)
