@@ -373,6 +373,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           for (int j = 0; j < 32; ++j)
             s[j] = mul2(make_float2(__uint_as_float(v[j >> 4][2 * (j & 15)]), __uint_as_float(v[j >> 4][2 * (j & 15) + 1])), sl22);
         }
+        if (!mine && ok) {                               // on their way first: the peer waits for them
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            st_async_f32x4(x_row + to_peer + j * (kHo * 16), smem_u32(&x_full[grp]) + to_peer, s[2 * j], s[2 * j + 1]);
+        }
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_free);
@@ -437,11 +442,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           l_run += sum.x + sum.y;
         } else {
           if ((quad & 1) == 0 && lane == 0) mbar_expect_tx(&px_full[grp], kPxBytes + kHo * 4);
-          if (ok) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              st_async_f32x4(x_row + to_peer + j * (kHo * 16), smem_u32(&x_full[grp]) + to_peer, s[2 * j], s[2 * j + 1]);
-          }
           if (!mbar_wait(&px_full[grp], use & 1, deadline)) ok = false;
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
@@ -535,7 +535,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (!ok && lane == 0) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
   } else if (warp >= kFirstDq) {
     // =========================== dequantisation ===========================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const int w8 = warp - kFirstDq;
     // Eight consecutive lanes (one phase of a 16-byte shared-memory access) hold four chunks of an even row and the
     // four of the odd row below: their swizzled stores fall in all eight 16-byte bank groups.
@@ -628,7 +628,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (!ok) atomicCAS(p.error_flag, 0, (int)kTimeoutMbarrier);
   } else {
     // =========================== MMA issue ===========================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    // 48, taken from the dequantisation warps, which do with 64: with 32 the issuing warp spilled, and a call of one tile per cluster
+    // (2 x 1500 tokens) took 26.6 us instead of 25.2
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     if (warp == 0) {
       constexpr uint32_t id_qk = umma_idesc_bf16(kH, kTile);
       constexpr uint32_t id_pv = umma_idesc_bf16(kH, kDo) | (1u << 16);       // B is MN-major
@@ -643,8 +645,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       // byte offsets enter a descriptor in 16-byte units and never carry out of its 14-bit address field
       auto qk = [&](uint32_t n_lane) {
         const uint32_t n = __shfl_sync(0xffffffffu, n_lane, 0);
-        if (!wait(&kv_full[n % kSlots], (n / kSlots) & 1)) return false;
-        if (n >= 1 && !wait(&s_free, (n - 1) & 1)) return false;
+        // both at once, a lane each: a wait that has nothing to wait for still takes ~200 cycles
+        bool good = true;
+        if (lane == 0) good = mbar_wait(&kv_full[n % kSlots], (n / kSlots) & 1, deadline);
+        else if (lane == 1 && n >= 1) good = mbar_wait(&s_free, (n - 1) & 1, deadline);
+        if (__all_sync(0xffffffffu, good) == 0) return false;
+        __syncwarp();                                    // what either lane has seen holds for the one that issues
         tc_fence_after_sync();
         const uint32_t slot = (n % kSlots) * kSlotBytes;
         if (elect_one()) {

@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lse_combine_half_kernel(con
     const float w = l == -INFINITY ? -1.f : exp2f(l - top);          // below zero: the row is not even read
     sum += fmaxf(w, 0.f);
     const int count = min(kHalf, p.n - n0);
+#pragma unroll 2
     for (int k = 0; k < count; ++k) {
       const float wk = __shfl_sync(kFull, w, k, kHalf);
       if (wk >= 0.f && lane < nchunks) {
