@@ -330,7 +330,10 @@ OprojForm oproj_form(int hidden, int K, int tokens, int64_t splits, bool packed,
     if (const char* v = std::getenv("HELIX_A2A_OPROJ_STREAMK")) f.streamk = std::string(v) == "1";
   }
   if (!f.streamk && (splits == 0 || (packed && splits < 0))) f.plan = helix::oproj_pick_split_plan(hidden, K, tokens, sms);
-  if (splits <= 0) f.splits = f.plan.slabs > 0 ? f.plan.splits : helix::oproj_pick_splits(hidden, K, sms);
+  if (splits <= 0)
+    f.splits = f.plan.slabs > 0 ? f.plan.splits
+               : tokens <= 8    ? helix::oproj_pick_splits_few(hidden, K, sms)
+                                : helix::oproj_pick_splits(hidden, K, sms);
   return f;
 }
 

@@ -35,6 +35,7 @@ inline size_t oproj_partial_bytes(int hidden, int splits, int n_pad) {
   return (size_t)(hidden / 128) * splits * n_pad * 128 * sizeof(float);
 }
 int oproj_pick_splits(int hidden, int K, int sm_count);
+int oproj_pick_splits_few(int hidden, int K, int sm_count);      // of the plain kernel, up to 8 tokens
 int oproj_pick_stages(int n_pad);
 int oproj_pick_atoms(int n_pad);
 int oproj_smem_bytes(int n_pad, int stages);

@@ -457,6 +457,20 @@ int oproj_pick_splits(int hidden, int K, int sm_count) {
   return std::min(splits, 8);
 }
 
+// Up to 8 tokens the fold of the splits is cheap, so what counts is whether the SMs are busy.  From K = 2048 on, few slabs (an eighth of
+// the SMs; at K = 2048 a quarter) take four splits although each then keeps only 512 of K; more slabs than a third of the SMs stay in
+// one piece at K = 2048.  Longer K keeps the general rule between the two: at K = 2560 the blocks of 256 no longer split evenly, and
+// 4096 and 5120 lost 2 to 3% with more splits, 7168 lost 5% with one.  Measured in a graph, plain weights, 8 tokens, before and after:
+// 1024 x 2048 9.9, 8.6 us; 1024 x 2560 10.7, 9.6; 2048 x 2048 10.3, 9.5; 2048 x 2560 11.0, 10.4; 4096 x 2048 11.3, 10.7;
+// 7168 x 2048 12.8, 12.5; 8192 x 2048 13.7, 13.1 (packed weights 12.7 both ways).
+int oproj_pick_splits_few(int hidden, int K, int sm_count) {
+  const int m_tiles = hidden / kBM, kb_total = (K + 255) / 256, general = oproj_pick_splits(hidden, K, sm_count);
+  if (kb_total < 8) return general;
+  if (m_tiles * 3 > sm_count) return kb_total == 8 ? 1 : general;
+  if (m_tiles * 8 <= sm_count || (m_tiles * 4 <= sm_count && kb_total == 8)) return std::max(general, 4);
+  return general;
+}
+
 int oproj_smem_bytes(int n_pad, int stages) {
   return stages * (kBM + n_pad) * kAtomK * oproj_pick_atoms(n_pad) * 2 + 1024;
 }
@@ -494,7 +508,9 @@ cudaError_t launch_oproj(const OprojParams& p, bool pdl, cudaStream_t stream) {
 }
 
 
-// Stream-K is picked only when the plain grid (slabs x splits) would leave more than a fifth of the SMs idle,
+// Stream-K is picked only when the plain grid (slabs x splits) would leave more than a quarter of the SMs idle (a fifth for more than
+// 16 tokens over more than 8192 of K; stream-K and plain, plain weights: 7168 x 8192 at 8 tokens 28.3 and 26.9 us, at 16 29.4 and 28.2,
+// at 31 32.5 and 31.5; 7168 x 16384 at 16 50.5 and 48.8, at 31 53.5 and 55.0; 4864 x 8192 at 16 23.3 and 22.9, at 31 26.5 and 24.0),
 // there are at least 8 units per CTA to deal out, and the token tile is small (the piece fold grows with
 // n_pad: at 256 tokens and K = 1024 it costs 51 us against 18 us plain).  With a fuller plain grid the two run
 // level (8192 x 8192 under programmatic launch: 128 plain CTAs 26.0 us, 148 stream-K CTAs 26.6 us).
@@ -502,7 +518,8 @@ bool oproj_streamk_pays(int hidden, int K, int n_pad, int sm_count) {
   const int bk = kAtomK * oproj_pick_atoms(n_pad);
   const long long units = (long long)(hidden / kBM) * ((K + bk - 1) / bk);
   const int plain_ctas = (hidden / kBM) * oproj_pick_splits(hidden, K, sm_count);
-  return n_pad <= 32 && plain_ctas * 5 < sm_count * 4 && units >= 8LL * sm_count;
+  const bool idle = n_pad <= 16 || K <= 8192 ? plain_ctas * 4 < sm_count * 3 : plain_ctas * 5 < sm_count * 4;
+  return n_pad <= 32 && idle && units >= 8LL * sm_count;
 }
 
 cudaError_t launch_oproj_streamk(const OprojParams& p, bool pdl, cudaStream_t stream) {
