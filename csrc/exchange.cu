@@ -78,6 +78,7 @@ KernelFn pick_combine(bool bf16) {
 struct Variant {
   KernelFn fn;
   int nit;
+  int ctas_per_sm;
 };
 
 Variant pick_variant(const ExchangeParams& p, int iters) {
@@ -90,15 +91,16 @@ Variant pick_variant(const ExchangeParams& p, int iters) {
   const int ranks = p.ranks_in_launch, per_channel = p.outer * p.inner / std::max(device_sm_count() / ranks, 1);
   const bool dense = ranks > 1 && (iters <= 1 || per_channel >= 64);
   if (p.mode == kModeCombine) {
-    if (iters <= 1) return {dense ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1};
-    if (iters <= 2) return {dense ? pick_combine<2, 2>(p.is_bf16) : pick_combine<2, 1>(p.is_bf16), 2};
-    if (iters <= 3) return {dense ? pick_combine<3, 2>(p.is_bf16) : pick_combine<3, 1>(p.is_bf16), 3};
-    if (iters <= 5) return {pick_combine<5, 1>(p.is_bf16), 5};
-    if (iters <= 9) return {pick_combine<9, 1>(p.is_bf16), 9};
-    return {nullptr, 0};
+    const int per_sm = dense ? 2 : 1;
+    if (iters <= 1) return {dense ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1, per_sm};
+    if (iters <= 2) return {dense ? pick_combine<2, 2>(p.is_bf16) : pick_combine<2, 1>(p.is_bf16), 2, per_sm};
+    if (iters <= 3) return {dense ? pick_combine<3, 2>(p.is_bf16) : pick_combine<3, 1>(p.is_bf16), 3, per_sm};
+    if (iters <= 5) return {pick_combine<5, 1>(p.is_bf16), 5, 1};
+    if (iters <= 9) return {pick_combine<9, 1>(p.is_bf16), 9, 1};
+    return {nullptr, 0, 0};
   }
-  if (iters <= 1) return {(KernelFn)helix_exchange_kernel<false, true, 1, 1>, 1};
-  return {(KernelFn)helix_exchange_kernel<false, true, 3, 1>, 3};  // larger messages go in slabs of 3
+  if (iters <= 1) return {(KernelFn)helix_exchange_kernel<false, true, 1, 1>, 1, 1};
+  return {(KernelFn)helix_exchange_kernel<false, true, 3, 1>, 3, 1};  // larger messages go in slabs of 3
 }
 
 size_t group_smem_bytes(int nit, int recv_warps, int group_warps) {
@@ -223,6 +225,15 @@ LaunchInfo plan_launch(const ExchangeParams& p, int channel_override) {
   return li;
 }
 
+// messages of the peers that one warp of a channel sends, or takes in, one after the other
+static int message_chain(const ExchangeParams& p, const LaunchInfo& li) {
+  const int peers = p.cp_size - 1, entries = ceil_div(p.outer * p.inner, li.channels);
+  const int send = ceil_div(entries * peers, li.send_warps);
+  const int recv = p.mode == kModeCombine ? ceil_div(entries, li.recv_warps / li.group_warps) * ceil_div(peers, li.group_warps)
+                                          : ceil_div(entries * p.cp_size, li.recv_warps);
+  return std::max(send, recv);
+}
+
 cudaError_t launch_exchange(ExchangeParams p, int channel_override, bool pdl, cudaStream_t stream,
                             LaunchInfo* info_out) {
   const int E = p.outer * p.inner;
@@ -241,13 +252,23 @@ cudaError_t launch_exchange(ExchangeParams p, int channel_override, bool pdl, cu
   int cap_channels = capacity / p.ranks_in_launch;
   if (cap_channels < 1) return cudaErrorLaunchOutOfResources;
   if (li.channels > cap_channels) {
-    // fewer channels, more entries for each: the split of its warps is chosen again
-    li = plan_launch(p, cap_channels);
-    threads = 32 * (li.send_warps + li.recv_warps);
-    smem = p.mode == kModeCombine ? group_smem_bytes(var.nit, li.recv_warps, li.group_warps) : 0;
-    capacity = resident_ctas(var.fn, threads, smem);
-    if (capacity < p.ranks_in_launch) return cudaErrorLaunchOutOfResources;
-    li.channels = std::min(li.channels, capacity / p.ranks_in_launch);
+    // Fewer channels, more entries for each: the split of its warps is chosen again.  Larger CTAs may halve the channels once
+    // more (two small ones share an SM); then the second plan has to shorten the longest chain of messages in a warp.  First
+    // and second plan, us: rows of 512, 5 ranks, 512 entries each 17.6 (59 channels) and 23.0 (29), 6 ranks, 362 entries
+    // 20.2 and 21.9, but rows of 1024, 8 ranks, 91 entries 37.6 and 27.7.  A third CTA gains nothing where two share an
+    // SM anyway: rows of 128, 4 ranks, 512 entries 12.3 (111 channels) and 10.8 (74).
+    LaunchInfo again = plan_launch(p, cap_channels);
+    const int again_threads = 32 * (again.send_warps + again.recv_warps);
+    const size_t again_smem = p.mode == kModeCombine ? group_smem_bytes(var.nit, again.recv_warps, again.group_warps) : 0;
+    const int again_channels = resident_ctas(var.fn, again_threads, again_smem) / p.ranks_in_launch;
+    again.channels = std::min(again.channels, again_channels);
+    li.channels = cap_channels;
+    const bool keeps = again.channels == cap_channels || var.ctas_per_sm > 1;
+    if (again_channels >= 1 && (keeps || message_chain(p, again) < message_chain(p, li))) {
+      li = again;
+      threads = again_threads;
+      smem = again_smem;
+    }
   }
 
   p.channels = li.channels;
