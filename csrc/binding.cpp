@@ -491,6 +491,7 @@ PYBIND11_MODULE(_C, m) {
     d["lines_per_message"] = li.lines_per_message;
     d["iters"] = li.iters;
     d["cooperative"] = li.cooperative;
+    d["ctas_per_sm"] = li.ctas_per_sm;
     return d;
   });
   m.def("layout", [](int cp, int sm_count) {

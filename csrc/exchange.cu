@@ -81,15 +81,20 @@ struct Variant {
   int ctas_per_sm;
 };
 
-Variant pick_variant(const ExchangeParams& p, int iters) {
+Variant pick_variant(const ExchangeParams& p, int iters, int lines) {
   // A launch that plays several ranks shares the SMs between them, and a rank has a ring for every SM: its warps are too
-  // few to hide the latency of one message at a time, so there is an instance with half of the registers, two CTAs per SM.
-  // Rows of 128 (one iteration) always take it; with longer ones it spills and pays from some 64 entries per channel on.
-  // One call, one CTA per SM -> two (the plan made again for the channels that fit in both), us: 64 heads of 128, 8 ranks, 32 / 128
-  // tokens 27.6 -> 16.3 / 54.1 -> 36.0; 128 heads of 512, 4 / 8 ranks, 128 tokens (110 entries a channel) 75.0 -> 64.8 / 140 -> 125,
-  // but 2 ranks, 32 tokens (28 a channel) 14.3 -> 16.6 and 8 ranks, 8 tokens 17.4 -> 21.0.
+  // few to hide the latency of one message at a time, so there is an instance with half of the registers, two CTAs per SM
+  // (one and two iterations fit them, three spill).  It pays once a channel has enough to do.  One call, one and two CTAs per SM, us:
+  //   rows of 128, messages of the peers per channel: 2 ranks 6 of them 5.1 and 5.5, 8 5.9 and 5.7; 4 ranks 3 5.3 and 6.0, 9 6.7 and 6.5;
+  //   7 ranks 6 6.6 and 6.9, 12 8.6 and 7.6; a call of 37 entries, 2 ranks, 4.4 and 4.9; 8 ranks, 56 entries a channel 44 and 34
+  //   rows of 256, entries per channel: 2 ranks 48 of them 14.7 and 14.8, 66 17.8 and 17.7; 4 ranks 66 32.9 and 30.3; 8 ranks
+  //   8 14.4 and 15.5, 17 21.6 and 23.3, 66 67 and 54; of 464: 2 ranks 48 14.8 and 15.3, 8 ranks 66 81 and 60
+  //   rows of 512 (9 lines), entries per channel times ranks: 2 ranks 150 of them 23.7 and 25.5, 200 30.5 and 31.6, 268 41.3 and 40.1;
+  //   3 ranks 200 29.9 and 32.1, 300 level; 4 ranks 200 32.7 and 32.5, 268 43.5 and 41.3; 8 ranks 240 39.6 and 40.1, 350 58.6 and 53.1;
+  //   of 704 (12 lines): 2 ranks 150 24.2 and 27.3, 268 52.0 and 49.0; 3 ranks 150 25.1 and 26.7, 200 34.8 and 34.4, 268 48.1 and 44.0
   const int ranks = p.ranks_in_launch, per_channel = p.outer * p.inner / std::max(device_sm_count() / ranks, 1);
-  const bool dense = ranks > 1 && (iters <= 1 || per_channel >= 64);
+  const bool pays = iters <= 1 ? per_channel * (ranks - 1) >= 8 : iters <= 2 ? per_channel >= 64 : per_channel * ranks * lines >= 2304;
+  const bool dense = ranks > 1 && pays;
   if (p.mode == kModeCombine) {
     const int per_sm = dense ? 2 : 1;
     if (iters <= 1) return {dense ? pick_combine<1, 2>(p.is_bf16) : pick_combine<1, 1>(p.is_bf16), 1, per_sm};
@@ -241,7 +246,7 @@ cudaError_t launch_exchange(ExchangeParams p, int channel_override, bool pdl, cu
   if (p.cp_size < 1 || p.cp_size > kMaxCp || p.ranks_in_launch < 1 || p.ranks_in_launch > kMaxEmulatedRanks)
     return cudaErrorInvalidValue;
   LaunchInfo li = plan_launch(p, channel_override);
-  Variant var = pick_variant(p, li.iters);
+  Variant var = pick_variant(p, li.iters, li.lines_per_message);
   if (var.fn == nullptr) return cudaErrorInvalidValue;
 
   int threads = 32 * (li.send_warps + li.recv_warps);
@@ -310,6 +315,7 @@ cudaError_t launch_exchange(ExchangeParams p, int channel_override, bool pdl, cu
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
+  li.ctas_per_sm = var.ctas_per_sm;
   if (info_out) *info_out = li;
   return cudaLaunchKernelEx(&cfg, var.fn, p);
 }

@@ -81,6 +81,7 @@ struct LaunchInfo {
   int lines_per_message;
   int iters;            // warp iterations per message (4 lines each)
   int cooperative;
+  int ctas_per_sm;      // that the launched kernel leaves registers for (0: planned, not launched)
 };
 
 int max_channel_count(int cp_size, int sm_count);            // rings per (row, sender)

@@ -41,3 +41,14 @@ def test_small_ctas_that_share_an_sm_keep_their_channels(native_built, cp, entri
 def test_larger_ctas_where_they_shorten_the_chain(native_built, cp, entries, dim, recv):
     info = _call(cp, entries, dim)
     assert info["channels"] * cp <= torch.cuda.get_device_properties(0).multi_processor_count and info["recv_warps"] == recv, info
+
+
+# on 148 SMs: messages of the peers per channel below and from 8 (rows of 128), entries per channel below and from 64 (rows of 256),
+# entries per channel times ranks times lines below and from 2304 (rows of 512, 9 lines, and of 704, 12 lines)
+@pytest.mark.parametrize("cp,entries,dim,ctas", [
+    (2, 32, 128, 1), (8, 16, 128, 1), (4, 64, 128, 1), (2, 591, 128, 1), (2, 592, 128, 2), (8, 36, 128, 2),
+    (2, 4735, 256, 1), (2, 4736, 256, 2), (8, 1152, 256, 2),
+    (2, 5920, 512, 1), (2, 9472, 512, 2), (3, 3136, 512, 1), (4, 2367, 512, 1), (4, 2368, 512, 2), (8, 576, 512, 2),
+    (3, 3087, 704, 1), (3, 3136, 704, 2)])
+def test_two_ctas_per_sm_where_a_channel_has_enough_to_do(native_built, cp, entries, dim, ctas):
+    assert _call(cp, entries, dim)["ctas_per_sm"] == ctas
