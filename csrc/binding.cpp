@@ -508,6 +508,7 @@ PYBIND11_MODULE(_C, m) {
     return d;
   });
   m.def("wire_bytes", [](int payload_bytes) { return helix::ll128::wire_bytes_for_words((payload_bytes + 7) / 8); });
+  m.def("lse_combine_half_warps", &helix::lse_combine_half_warps);
   // what the auto-tuner would choose for a call (no launch, no GPU): entries = outer * inner rows of o_bytes + stats
   m.def("plan_info", [](int cp, int sm_count, int outer, int inner, int o_bytes, int st_words, bool combine) {
     helix::ExchangeParams p{};

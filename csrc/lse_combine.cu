@@ -6,8 +6,9 @@
 // rank's rows: users of the plain `alltoall`, and the NCCL path of the vLLM hook.  Counterpart of the
 // reference's Triton kernel (patches/dcp_alltoall_helix.py:210-384), with its rules: NaN and +-inf LSEs count
 // as -inf (no contribution), a row whose LSEs are all -inf comes out as zeros with a global LSE of -inf,
-// base e or base 2.  One warp per row (half a warp for short ones), the online accumulator of the exchange's receive side in registers,
-// 16-byte loads; a row is read once and never staged.
+// base e or base 2.  One warp per row with the online accumulator of the exchange's receive side in registers, or, for short rows,
+// half a warp that takes the maximum of the row's LSEs first and then adds up weighted rows (LSEs beyond the sixteenth rank are read
+// twice).  16-byte loads; a row is read once and never staged.
 #include "lse_combine.h"
 
 #include "exchange_device.cuh"
@@ -77,7 +78,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lse_combine_kernel(const __
 // ranks' LSEs, so that a rank costs a row eight multiply-adds per lane and no exponential.  The kernel above is bound by its
 // instructions there: 16384 rows of 128, 8 / 4 / 2 ranks (in a graph) 17.8 / 9.0 / 6.5 -> 13.4 / 5.6 / 4.6 us, 2048 rows 5.0 / 3.4 / 2.7
 // -> 4.0 / 3.2 / 2.7.  For rows of 512 it is the other way round: the same arithmetic with a warp per row took 35.7 us against
-// 30.6 (8 ranks, 16384 rows), and with two or four ranks' rows in flight at once 35.9 and 42.7.
+// 30.6 (8 ranks, 16384 rows), and with two or four ranks' rows in flight at once 35.9 and 42.7.  One or two ranks below 2048 rows
+// keep a warp per row too (lse_combine_half_warps).
 constexpr int kHalf = 16;
 template <bool BF16>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) lse_combine_half_kernel(const __grid_constant__ LseCombineParams p) {
@@ -153,15 +155,25 @@ Fn pick(bool bf16) {
 
 }  // namespace
 
+// Half a warp per row reduces the LSEs over the lanes before the first row is on its way, about 0.2 us.  With one or two ranks and
+// few rows nothing makes up for it.  Rows of 128, a warp and half a warp per row, in a graph, us: 1 rank 128 rows 1.84 and 1.99, 2048
+// rows 2.05 and 2.15, 4096 rows level; 2 ranks 4 rows 1.92 and 2.09, 1024 rows 2.35 and 2.37 (2.21 and 2.33 where a row's LSEs lie
+// together), 2048 rows level, 4096 rows 2.73 and 2.57; 3 ranks 128 rows 2.62 and 2.45 (2.37 and 2.44 there).  The layout is left
+// out of the rule, so that both give the same bits.
+bool lse_combine_half_warps(int64_t rows, int n, int row_bytes) {
+  return row_bytes <= kHalf * 16 && (n > 2 || rows >= 2048);
+}
+
 cudaError_t launch_lse_combine(const LseCombineParams& p, bool pdl, cudaStream_t stream) {
   if (p.rows <= 0 || p.n <= 0) return cudaSuccess;
   if (p.row_bytes <= 0 || p.row_bytes % 16 != 0 || p.row_bytes > 4 * 32 * 16) return cudaErrorInvalidValue;
   const int chunks = p.row_bytes / 16;
-  Fn fn = chunks <= kHalf ? (p.is_bf16 ? (Fn)lse_combine_half_kernel<true> : (Fn)lse_combine_half_kernel<false>)
+  const bool half = lse_combine_half_warps(p.rows, p.n, p.row_bytes);
+  Fn fn = half            ? (p.is_bf16 ? (Fn)lse_combine_half_kernel<true> : (Fn)lse_combine_half_kernel<false>)
           : chunks <= 32  ? pick<1>(p.is_bf16)
           : chunks <= 64  ? pick<2>(p.is_bf16)
                           : pick<4>(p.is_bf16);
-  const int rows_per_cta = chunks <= kHalf ? 2 * kWarpsPerCta : kWarpsPerCta;
+  const int rows_per_cta = half ? 2 * kWarpsPerCta : kWarpsPerCta;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((p.rows + rows_per_cta - 1) / rows_per_cta), 1, 1);
   cfg.blockDim = dim3(kWarpsPerCta * 32, 1, 1);

@@ -19,6 +19,9 @@ struct LseCombineParams {
   int base2;              // LSEs are base 2 (else base e); the global LSE comes out in the same base
 };
 
+// whether a call's rows take half a warp each (else a warp)
+bool lse_combine_half_warps(int64_t rows, int n, int row_bytes);
+
 cudaError_t launch_lse_combine(const LseCombineParams& p, bool pdl, cudaStream_t stream);
 
 }  // namespace helix

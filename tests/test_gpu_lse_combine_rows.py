@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 # rows that end inside a warp and a block; both sides of the 16-chunk rule (128 elements)
 @pytest.mark.parametrize("n,rows,dim", [(1, 1, 8), (2, 7, 64), (3, 17, 128), (8, 33, 128), (9, 5, 136), (16, 8, 120), (17, 4, 128),
-                                        (33, 3, 128), (40, 9, 512), (4, 2, 520)])
+                                        (33, 3, 128), (40, 9, 512), (4, 2, 520), (2, 2047, 128), (2, 2048, 128), (2, 2049, 72)])
 @pytest.mark.parametrize("layout", ["NBHD", "BHND"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_combine_rows(native_built, n, rows, dim, layout, dtype):
