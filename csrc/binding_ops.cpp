@@ -628,6 +628,7 @@ void register_compute_ops(torch::Library& m) {
 void bind_compute(pybind11::module_& m) {
   m.def("gqa_pick_ctas", &helix::gqa_pick_ctas);
   m.def("oproj_pick_splits", &helix::oproj_pick_splits);
+  m.def("oproj_pick_splits_few", &helix::oproj_pick_splits_few);
   m.def("gqa_launches", &gqa_launches);
   m.def("oproj_launches", &oproj_launches);
   m.def("fused_oproj_fits", &fused_oproj_fits);

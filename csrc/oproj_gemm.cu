@@ -457,18 +457,26 @@ int oproj_pick_splits(int hidden, int K, int sm_count) {
   return std::min(splits, 8);
 }
 
-// Up to 8 tokens the fold of the splits is cheap, so what counts is whether the SMs are busy.  From K = 2048 on, few slabs (an eighth of
-// the SMs; at K = 2048 a quarter) take four splits although each then keeps only 512 of K; more slabs than a third of the SMs stay in
-// one piece at K = 2048.  Longer K keeps the general rule between the two: at K = 2560 the blocks of 256 no longer split evenly, and
-// 4096 and 5120 lost 2 to 3% with more splits, 7168 lost 5% with one.  Measured in a graph, plain weights, 8 tokens, before and after:
-// 1024 x 2048 9.9, 8.6 us; 1024 x 2560 10.7, 9.6; 2048 x 2048 10.3, 9.5; 2048 x 2560 11.0, 10.4; 4096 x 2048 11.3, 10.7;
-// 7168 x 2048 12.8, 12.5; 8192 x 2048 13.7, 13.1 (packed weights 12.7 both ways).
+// Up to 8 tokens the fold of the splits is cheap, so what counts is whether the SMs are busy.  A split takes whole blocks of 256.
+// From K = 1793 (eight blocks) on, few slabs (an eighth of the SMs; with eight blocks a quarter) take four splits, of two or
+// three blocks up to twelve; more slabs than a third of the SMs stay in one piece with eight blocks.  Longer K keeps the general rule
+// between the two: at K = 2560 4096 and 5120 rows lost 2 to 3% with more splits, 7168 lost 5% with one.  A count that leaves
+// its last split without a block (nine blocks in four) is cut to the splits that have one.  In a graph, 8 tokens, us, by the general
+// rule and now, plain weights (packed ones within 0.1): 1024 x 2048 10.0, 8.6; 1024 x 2304 10.9, 9.3 (9.8 in four); 1024 x 2560
+// 10.8, 9.75; 2048 x 1856 10.1, 9.1; 2304 x 2816 11.9, 10.7; 4096 x 2048 11.1, 10.4; 4736 x 1856 11.3, 10.5; 8192 x 2048 13.2, 12.5.
+// From 50 to 60 slabs the two sides of the last line are within 2% of one another, ahead by turns (6400 x 1856 11.8 in two, 12.0 in
+// one; 7168 x 2048 12.4 and 12.2).
 int oproj_pick_splits_few(int hidden, int K, int sm_count) {
-  const int m_tiles = hidden / kBM, kb_total = (K + 255) / 256, general = oproj_pick_splits(hidden, K, sm_count);
-  if (kb_total < 8) return general;
-  if (m_tiles * 3 > sm_count) return kb_total == 8 ? 1 : general;
-  if (m_tiles * 8 <= sm_count || (m_tiles * 4 <= sm_count && kb_total == 8)) return std::max(general, 4);
-  return general;
+  const int m_tiles = hidden / kBM, kb_total = (K + 255) / 256;
+  int splits = oproj_pick_splits(hidden, K, sm_count);
+  if (kb_total < 8) return splits;
+  if (m_tiles * 3 > sm_count) {
+    if (kb_total == 8) splits = 1;
+  } else if (m_tiles * 8 <= sm_count || (m_tiles * 4 <= sm_count && kb_total == 8)) {
+    splits = std::max(splits, 4);
+  }
+  const int per_split = (kb_total + splits - 1) / splits;
+  return (kb_total + per_split - 1) / per_split;
 }
 
 int oproj_smem_bytes(int n_pad, int stages) {

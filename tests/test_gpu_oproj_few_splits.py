@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("hidden,K,tokens", [
     (1024, 1792, 8), (1024, 1856, 8), (2048, 2048, 1), (2048, 2048, 9), (2304, 2560, 8), (4096, 2048, 8), (4736, 2048, 8),
     (4096, 2112, 3), (6272, 2048, 8), (6400, 2048, 8), (8192, 2048, 1), (8192, 2304, 8), (7168, 8192, 8), (7168, 8192, 17),
-    (4864, 8192, 16), (4864, 8256, 32)])
+    (4864, 8192, 16), (4864, 8256, 32), (1024, 2304, 8), (2048, 2112, 1), (2304, 6400, 8)])
 @pytest.mark.parametrize("packed", [False, True])
 def test_few_tokens_match_fp32(native_built, hidden, K, tokens, packed):
     from helix_a2a_b200.ops import oproj as O
