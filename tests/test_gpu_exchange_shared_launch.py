@@ -52,3 +52,18 @@ def test_larger_ctas_where_they_shorten_the_chain(native_built, cp, entries, dim
     (3, 3087, 704, 1), (3, 3136, 704, 2)])
 def test_two_ctas_per_sm_where_a_channel_has_enough_to_do(native_built, cp, entries, dim, ctas):
     assert _call(cp, entries, dim)["ctas_per_sm"] == ctas
+
+
+# Rows of one, two and three iterations on two CTAs per SM.  Messages of 3, 5 and 9 lines: 342 entries a channel of rows of 128, 206 of
+# rows of 256 and 115 of rows of 512 are more than half a ring of 2048, so receivers publish within the call, and three calls go
+# round the ring.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cp,entries,dim", [
+    (2, 148 * 345 + 3, 128), (4, 74 * 345 + 3, 128), (8, 37 * 345 + 3, 128),
+    (2, 148 * 210 + 5, 256), (4, 37 * 64, 256), (8, 18 * 70 + 1, 256), (3, 98 * 210 + 1, 240),
+    (2, 74 * 230 + 7, 512), (4, 37 * 66, 512)])
+def test_bulk_calls_on_two_ctas_per_sm(native_built, dtype, cp, entries, dim):
+    info = _call(cp, entries, dim, dtype, calls=3)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert info["ctas_per_sm"] == 2 and info["channels"] * cp > sms, info
+    assert info["recv_warps"] > 8 and info["send_warps"] + info["recv_warps"] <= 16, info      # the bulk split of a CTA's warps
