@@ -39,7 +39,7 @@ def gqa_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bl
     if max_seq_len <= 0:
         max_seq_len = block_table.shape[1] * (k_cache.shape[2] if layout == "HND" else k_cache.shape[1])
     return _ext.ops().gqa_decode(q, k_cache, v_cache, block_table, seq_lens, float(scale), lse_base2,
-                            layout == "HND", splits, max_seq_len, kv_stable)
+                                 layout == "HND", splits, max_seq_len, kv_stable)
 
 
 def mla_decode(q_nope: torch.Tensor, q_pe: torch.Tensor, ckv_fp8: torch.Tensor, scales: torch.Tensor,
@@ -72,4 +72,4 @@ def mla_decode(q_nope: torch.Tensor, q_pe: torch.Tensor, ckv_fp8: torch.Tensor, 
     if max_seq_len <= 0:
         max_seq_len = block_table.shape[1] * ckv_fp8.shape[1]
     return _ext.ops().mla_decode(q_nope, q_pe, ckv_fp8, scales, kpe, block_table, seq_lens, float(scale), lse_base2,
-                            ctas, max_seq_len)
+                                 ctas, max_seq_len)
